@@ -13,7 +13,8 @@
 //   4. records  : one thread per unique row resolves everything the update needs
 //                 (row address, first gradient row address, run, width) into a
 //                 32-byte record; runs longer than C reserve chunk slots.
-//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp).
+//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp), and for runs of
+//                 many chunks the total of those.
 //   5. update   : G lanes per unique row: record (fetched one row ahead) -> w / m1 /
 //                 m2 / first gradient row in one wave of loads -> remaining gradient
 //                 rows or chunk sums in order -> optimizer -> one write of w / m1 /
@@ -28,6 +29,8 @@
 #ifndef RECSDK_EMULATE
 namespace recsdk {
 // ---------------------------------------------------------------------------- host side
+constexpr int64_t kLongRunMinIds = 32768;
+
 struct BwdWorkspace {
     void *keys_a, *keys_b;
     uint32_t *vals_a, *vals_b, *sort_scratch;
@@ -35,6 +38,7 @@ struct BwdWorkspace {
     RunMeta* meta;
     int2* desc;
     float* partial;
+    int* long_list;
     int64_t* counters;
     size_t bytes;
 };
@@ -56,6 +60,7 @@ static BwdWorkspace carve_bwd(void* base, int64_t N, int32_t max_D)
     w.desc = c.take<int2>(max_chunks);
     w.scan_scratch = c.take<int>(scan_scratch_ints(N));
     w.partial = c.take<float>(max_chunks * static_cast<size_t>(max_D));
+    w.long_list = c.take<int>(long_runs_cap(N));
     w.bytes = c.used();
     return w;
 }
@@ -119,8 +124,9 @@ template <int G, int K>
 static void launch_partial(const BwdParams& p, int64_t N, cudaStream_t st)
 {
     const int groups_per_block = 256 / G;
-    // one resident wave (64 registers under the launch bounds: 4 blocks per SM)
-    const int grid = grid_for(static_cast<int64_t>(chunk_slots_cap(N)), groups_per_block, 4);
+    // four waves of resident blocks: how many chunks there are is known on the device only, and a grid that is no
+    // multiple of the resident blocks leaves SMs idle behind the last wave
+    const int grid = grid_for(static_cast<int64_t>(chunk_slots_cap(N)), groups_per_block, 4 * chunk_blocks(G));
     partial_kernel<G, K><<<grid, 256, 0, st>>>(p);
 }
 
@@ -160,6 +166,9 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     p.counters = ws.counters;
     p.chunk_desc = ws.desc;
     p.partial = ws.partial;
+    // below this many ids even one row that holds them all has a chain of a few dozen rounds: not worth a launch
+    p.long_chunks = (N >= kLongRunMinIds && p.chunk > 0) ? kLongChunks : 0;
+    p.long_list = ws.long_list;
     const int vec_per_row = (a->max_D + 3) / 4;
     if (do_plan) {
         // The plan needs the indices and the LAYOUT of the gradient, not the gradient: it can run ahead, on
@@ -191,6 +200,8 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
         RECSDK_DISPATCH_GK(vec_per_row, CALL_PARTIAL);
 #undef CALL_PARTIAL
     }
+    // 4c. totals of the runs with many chunks
+    if (p.long_chunks > 0) long_run_kernel<<<num_sms() * 6, kLongWarps * 32, 0, st>>>(p, ws.meta);
     // 5. update
     if (a->ev_update_start) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_update_start), st);
 #define CALL_UPDATE(G, K) launch_update<G, K>(p, ws.meta, N, st)
@@ -274,7 +285,7 @@ extern "C" int recsdk_tbe_backward(const recsdk_tbe_backward_args* a, void* stre
     p.opt = a->optimizer;
     p.bshift = bshift;
     p.chunk = a->reduce_chunk;
-    p.direct_max = kDirectMax;
+    p.direct_max = direct_max_for(a->N);
     p.lr = a->learning_rate;
     p.eps = a->eps;
     p.beta1 = a->beta1;

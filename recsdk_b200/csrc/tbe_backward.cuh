@@ -40,19 +40,35 @@
 namespace recsdk {
 
 constexpr int kChunk = 64;  // the only non-zero reduce_chunk supported
-// Runs of more than kDirectMax positions are summed by the chunk-sum kernel (lanes resolve the gradient rows of a
-// chunk in parallel and keep eight row loads in flight), the row-update kernel then reads one partial row per
-// chunk; shorter runs are summed inside the row-update kernel.  This routing does not touch the arithmetic: a run
-// of at most reduce_chunk positions is ONE chunk, and 0.0f + (its sequential sum) is that sum bit for bit (with
-// reduce_chunk 0 a longer run is one chunk as a whole).  Measured on the benchmark step with thresholds 8, 16, 32
-// and 64: within 2 % of each other, so the threshold is the chunk length.
+// Runs of more than direct_max positions are summed by the chunk-sum kernel (lanes resolve the gradient rows of a
+// chunk in parallel and keep eight or more row loads in flight), the row-update kernel then reads one partial row per
+// chunk; shorter runs are summed inside the row-update kernel, four rows at a time.  This routing does not touch the
+// arithmetic: a run of at most reduce_chunk positions is ONE chunk, and 0.0f + (its sequential sum) is that sum bit for
+// bit (with reduce_chunk 0 a longer run is one chunk as a whole).
+// Large batches hide the row update's chain behind other rows: thresholds 8, 16, 32 and 64 are within 2 % of each
+// other on the benchmark step, and 64 needs the smallest partial buffer.  Below kDirectSmallN ids the chain of the
+// longest direct run is what the kernel takes: 11 tables of 8..128 floats, 330 K ids, MEAN: 70 us with 64,
+// 47 with 8 (and the chunk sums 15 and 24).
 constexpr int kDirectMax = kChunk;
-// Slots of the partial buffer / chunk descriptors that n index positions can need.
+constexpr int kDirectMaxSmall = 8;
+constexpr int64_t kDirectSmallN = int64_t(1) << 20;
+static inline int direct_max_for(int64_t n) { return n <= kDirectSmallN ? kDirectMaxSmall : kDirectMax; }
+// Slots of the partial buffer / chunk descriptors that n index positions, or any smaller number of them, can need (a
+// workspace sized for the largest batch serves every smaller one).
 static inline size_t chunk_slots_cap(int64_t n)
 {
     const size_t m = static_cast<size_t>(n > 0 ? n : 1);
-    return m / kChunk + m / (kDirectMax + 1) + 2;
+    const size_t few = m < static_cast<size_t>(kDirectSmallN) ? m : static_cast<size_t>(kDirectSmallN);
+    const size_t small = few / kChunk + few / (kDirectMaxSmall + 1), large = m / kChunk + m / (kDirectMax + 1);
+    return (small > large ? small : large) + 2;
 }
+// Above this many chunks the sum over a run's chunk sums gets a kernel of its own (long_run_kernel).  The order of that
+// sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update keeps four in flight
+// beside its table row, a warp of that kernel 224.  Hottest row of 20 M Zipf(1.2) ids in 26 tables, about 2600 chunks:
+// the row update as a whole took 1027 us with its chain in it, 724 without, and this kernel 60.
+constexpr int kLongChunks = 64;
+// Runs that can be longer than that: n positions hold at most n / (kLongChunks * kChunk) of them.
+static inline size_t long_runs_cap(int64_t n) { return static_cast<size_t>(n > 0 ? n : 0) / (kLongChunks * kChunk) + 1; }
 // Chunks of a run of `len` positions that went through the chunk-sum kernel.
 __host__ __device__ __forceinline__ int chunks_of_run(int len, int chunk) { return chunk > 0 ? (len + chunk - 1) / chunk : 1; }
 
@@ -91,6 +107,10 @@ struct BwdParams {
     // (buffer number << kLocShardShift) | element offset inside that buffer; the buffers may be peer mappings.
     float* dst_ptrs[RECSDK_MAX_SHARDS];
     int32_t direct_max;  // runs longer than this go through the chunk-sum kernel (>= kDirectMax)
+    // > 0: runs of more than this many chunks are listed in long_list (counters[4] of them) and long_run_kernel leaves
+    // their total in their first chunk slot before the row update reads it
+    int32_t long_chunks;
+    int* __restrict__ long_list;
 };
 
 // Internal "optimizer" of the row-update kernels: no table is read, the summed gradient of the row is stored.
@@ -279,10 +299,85 @@ __device__ __forceinline__ float prep_grad(const BwdParams& p, float g, float sc
     return g;
 }
 
-// Sum of the gradient rows of sorted positions [s, e), columns (cb+lane+k*G) (in
-// V::W-element vectors), in position order starting from zero.
-template <typename V, int G, int K>
+template <int G>
+__device__ __forceinline__ unsigned group_mask()
+{
+    if (G == 32) return kFullMask;
+    return ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
+}
+
+// Sum of the gradient rows of sorted positions [s, e), columns (cb+lane+k*G) (in V::W-element vectors), in position
+// order starting from what `acc` holds.  The G lanes resolve RT tags each -- G * RT tags at once, one round of loads
+// for all of them -- and the group then walks the rows in order with U independent row loads in flight per lane.
+// Called by all lanes of a group with the same arguments.  RT * G is a multiple of U.
+template <typename V, int G, int K, int RT, int U>
 __device__ __forceinline__ void sum_grad_rows(const BwdParams& p, int s, int e, int cb, int lane, int nvec,
+                                              typename V::T (&acc)[K])
+{
+    constexpr int S = G * RT;
+    constexpr int kStep = U < G ? U : G;     // rows per lane set of one register of tags
+    constexpr int kRegs = U > G ? U / G : 1;  // registers of tags a step of U rows spans
+    static_assert(S % U == 0 && RT % kRegs == 0, "tags per round");
+    const unsigned gmask = group_mask<G>();
+    const bool mean = p.mode == RECSDK_POOL_MEAN;
+    uint32_t tag[RT];
+#pragma unroll
+    for (int r = 0; r < RT; ++r) tag[r] = s + r * G + lane < e ? p.vals[s + r * G + lane] : 0u;
+    for (int base = s; base < e; base += S) {
+        const float* ptr[RT];
+        float scale[RT];
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+            GradRow g;
+            g.ptr = nullptr;
+            g.scale = 1.0f;
+            if (base + r * G + lane < e) g = grad_row_of(p, tag[r]);
+            ptr[r] = g.ptr;
+            scale[r] = g.scale;
+            // the next round's tags travel while this round's rows do
+            const int next = base + S + r * G + lane;
+            tag[r] = next < e ? p.vals[next] : 0u;
+        }
+        const int cnt = e - base < S ? e - base : S;
+#pragma unroll
+        for (int r0 = 0; r0 < RT; r0 += kRegs) {
+#pragma unroll 1
+            for (int j0 = 0; j0 < G; j0 += kStep) {
+                const int q0 = r0 * G + j0;
+                if (q0 >= cnt) break;
+                typename V::T v[U][K];
+                float sc[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = r0 + u / kStep;  // u < kStep unless one step spans several registers of tags
+                    const int src = j0 + u % kStep;
+                    const float* gp = reinterpret_cast<const float*>(
+                        __shfl_sync(gmask, reinterpret_cast<unsigned long long>(ptr[r]), src, G));
+                    sc[u] = mean ? __shfl_sync(gmask, scale[r], src, G) : 1.0f;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const int c = cb + lane + k * G;
+                        v[u][k] = (q0 + u < cnt && c < nvec) ? V::ld_stream(gp + V::W * c) : V::zero();
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (q0 + u < cnt) {
+                        const float x_scale = sc[u];
+#pragma unroll
+                        for (int k = 0; k < K; ++k)
+                            acc[k] = add4(acc[k], map4(v[u][k], [&](float x) { return prep_grad(p, x, x_scale); }));
+                    }
+            }
+        }
+    }
+}
+
+// Sum of the gradient rows of sorted positions [s, e), columns (cb+lane+k*G) (in
+// V::W-element vectors), in position order starting from what `acc` holds.  For the short runs of the row update: every
+// lane reads the tags itself, which needs the fewest registers beside the row that is being updated.
+template <typename V, int G, int K>
+__device__ __forceinline__ void sum_short_run(const BwdParams& p, int s, int e, int cb, int lane, int nvec,
                                               typename V::T (&acc)[K])
 {
     int i = s;
@@ -338,21 +433,26 @@ __device__ __forceinline__ bool vec_ok_for(const BwdParams& p, int64_t wofs, int
 }
 
 // ---------------------------------------------------------------------------- 4b. chunk sums
-template <typename V, int G, int K>
-__device__ __forceinline__ void partial_body(const BwdParams& p, int c, int lane)
+// Narrow rows (G <= 8): eight tags per lane and 16 row loads in flight, two blocks per SM.  Wide rows: one tag per
+// lane, eight row loads, four blocks (64 registers) -- there the warps provide the bytes in flight, and 64-float rows
+// took 787 us with four tags per lane and three blocks against 612 with four.
+template <int G>
+__host__ __device__ constexpr int chunk_tags()
 {
-    const int2 be = p.chunk_desc[c];
-    const int p0 = be.x, e = be.y;
-    int32_t D;
-    int64_t wofs, f;
-    run_geometry(p, p.vals[p0], D, wofs, f);
+    return G == 1 ? 16 : (G <= 8 ? 8 : 1);
+}
+__host__ __device__ constexpr int chunk_blocks(int G) { return G <= 8 ? 2 : 4; }
+__host__ __device__ constexpr int chunk_loads(int G) { return G <= 8 ? 16 : 8; }
+
+template <typename V, int G, int K, int U>
+__device__ __forceinline__ void partial_body(const BwdParams& p, int2 be, float* out, int lane, int32_t D)
+{
     const int nvec = D / V::W;
-    float* out = p.partial + static_cast<int64_t>(c) * p.max_D;
     for (int cb = 0; cb < nvec; cb += G * K) {
         typename V::T acc[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = V::zero();
-        sum_grad_rows<V, G, K>(p, p0, e, cb, lane, nvec, acc);
+        sum_grad_rows<V, G, K, chunk_tags<G>(), U>(p, be.x, be.y, cb, lane, nvec, acc);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int col = cb + lane + k * G;
@@ -361,75 +461,27 @@ __device__ __forceinline__ void partial_body(const BwdParams& p, int c, int lane
     }
 }
 
-template <int G>
-__device__ __forceinline__ unsigned group_mask();
-
-// Chunk sums.  One group per chunk (<= kChunk sorted positions of one long run):
-// lanes resolve G gradient tags at a time to addresses in parallel, then the group
-// walks them in order with several independent 128-bit loads in flight.
+// Chunk sums.  One group per chunk (<= kChunk sorted positions of one long run).  Bound by the latency of its loads
+// when the batch is small (tag -> row, then the rows) and by L2 when it is large.  Resolving G tags, summing their
+// rows, resolving the next G was a chain of 16 such rounds for 16-float rows: 28 us for 4096 ids, however few.
+// Rows that are not on 16 bytes are read word by word, four words per lane (the bytes in flight of the other path).
 template <int G, int K>
-__global__ void __launch_bounds__(256, 4) partial_kernel(BwdParams p)
+__global__ void __launch_bounds__(256, chunk_blocks(G)) partial_kernel(BwdParams p)
 {
     const int groups_per_block = blockDim.x / G;
     const int lane = threadIdx.x % G;
-    const unsigned gmask = group_mask<G>();
     const int64_t total = p.counters[1];
-    constexpr int kUnroll = 8 / K;
     for (int64_t c = static_cast<int64_t>(blockIdx.x) * groups_per_block + threadIdx.x / G; c < total;
          c += static_cast<int64_t>(gridDim.x) * groups_per_block) {
         int32_t D;
         int64_t wofs, f;
         const int2 be = p.chunk_desc[c];
         run_geometry(p, p.vals[be.x], D, wofs, f);
-        if (vec_ok_for(p, wofs, D, f)) {
-            const int nvec = D >> 2;
-            float* out = p.partial + c * p.max_D;
-            for (int cb = 0; cb < nvec; cb += G * K) {
-                float4 acc[K];
-#pragma unroll
-                for (int k = 0; k < K; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int base = be.x; base < be.y; base += G) {
-                    const int pos = base + lane;
-                    GradRow g_l;
-                    g_l.ptr = nullptr;
-                    g_l.scale = 1.0f;
-                    if (pos < be.y) g_l = grad_row_of(p, p.vals[pos]);
-                    const int cnt = (be.y - base) < G ? (be.y - base) : G;
-                    for (int jj0 = 0; jj0 < cnt; jj0 += kUnroll) {
-                        float4 v[kUnroll][K];
-                        float sc[kUnroll];
-#pragma unroll
-                        for (int u = 0; u < kUnroll; ++u) {
-                            const int jj = jj0 + u;
-                            const int src = jj < cnt ? jj : 0;
-                            const float* gp = reinterpret_cast<const float*>(
-                                __shfl_sync(gmask, reinterpret_cast<unsigned long long>(g_l.ptr), src, G));
-                            sc[u] = __shfl_sync(gmask, g_l.scale, src, G);
-#pragma unroll
-                            for (int k = 0; k < K; ++k) {
-                                const int col = cb + lane + k * G;
-                                v[u][k] = (jj < cnt && col < nvec) ? ld_f4_stream(gp + 4 * col)
-                                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < kUnroll; ++u)
-                            if (jj0 + u < cnt) {
-                                const float s = sc[u];
-#pragma unroll
-                                for (int k = 0; k < K; ++k)
-                                    acc[k] = add4(acc[k], map4(v[u][k], [&](float x) { return prep_grad(p, x, s); }));
-                            }
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const int col = cb + lane + k * G;
-                    if (col < nvec) st_f4(out + 4 * col, acc[k]);
-                }
-            }
-        } else
-            partial_body<V1, G, K>(p, static_cast<int>(c), lane);
+        float* out = p.partial + c * p.max_D;
+        if (vec_ok_for(p, wofs, D, f))
+            partial_body<V4, G, K, chunk_loads(G) / K>(p, be, out, lane, D);
+        else
+            partial_body<V1, G, 4, 4>(p, be, out, lane, D);
     }
 }
 
@@ -530,6 +582,8 @@ __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* 
                                                         static_cast<unsigned long long>(c)));
             atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), static_cast<unsigned long long>(len));
             m.chunk_base = base;
+            if (p.long_chunks > 0 && c > p.long_chunks)
+                p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(counters + 4), 1ull)] = static_cast<int>(r);
             for (int k = 0; k < c; ++k) {
                 const int b0 = rs + k * step;
                 desc[base + k] = make_int2(b0, b0 + step < re ? b0 + step : re);
@@ -538,6 +592,51 @@ __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* 
         meta[r] = m;
     }
 }
+
+#ifndef RECSDK_EMULATE
+// ---------------------------------------------------------------------------- 4c. totals of the longest runs
+// One warp per (listed run, 32 columns): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
+// place of the run's first chunk sum (no other warp reads these columns of this run).  The chunk sums come through a
+// ring of kLongStages shared-memory stages of 32 rows, filled by asynchronous copies, so 224 rows are in flight
+// whatever the registers; each lane copies and reads its own column, so a stage needs no barrier.
+constexpr int kLongStages = 8;
+constexpr int kLongRows = 32;
+constexpr int kLongWarps = 1;
+static __global__ void __launch_bounds__(kLongWarps * 32) long_run_kernel(BwdParams p, const RunMeta* __restrict__ meta)
+{
+    __shared__ float ring[kLongWarps][kLongStages][kLongRows][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slabs = (p.max_D + 31) / 32;
+    const int64_t items = p.counters[4] * slabs;
+    for (int64_t w = static_cast<int64_t>(blockIdx.x) * kLongWarps + warp; w < items;
+         w += static_cast<int64_t>(gridDim.x) * kLongWarps) {
+        const RunMeta* m = meta + p.long_list[w / slabs];
+        const int col = static_cast<int>(w % slabs) * 32 + lane;
+        if (col >= (m->D & (kMetaVecBit - 1))) continue;
+        const int nc = chunks_of_run(m->len, p.chunk);
+        float* q = p.partial + static_cast<int64_t>(m->chunk_base) * p.max_D + col;
+        auto fill = [&](int c0) {
+            float(*st)[32] = ring[warp][(c0 / kLongRows) % kLongStages];
+#pragma unroll
+            for (int u = 0; u < kLongRows; ++u)
+                if (c0 + u < nc) cp_async_4(&st[u][lane], q + static_cast<int64_t>(c0 + u) * p.max_D);
+            cp_async_commit();  // a group per stage, empty ones included, so that the waits below can count them
+        };
+        for (int g = 0; g < kLongStages - 1; ++g) fill(g * kLongRows);
+        float acc = 0.f;
+        for (int c0 = 0; c0 < nc; c0 += kLongRows) {
+            fill(c0 + (kLongStages - 1) * kLongRows);
+            cp_async_wait<kLongStages - 1>();
+            float(*st)[32] = ring[warp][(c0 / kLongRows) % kLongStages];
+#pragma unroll
+            for (int u = 0; u < kLongRows; ++u)
+                if (c0 + u < nc) acc = __fadd_rn(acc, st[u][lane]);
+        }
+        cp_async_wait<0>();
+        *q = acc;
+    }
+}
+#endif  // RECSDK_EMULATE
 
 // ---------------------------------------------------------------------------- 5b. row update
 // Summed gradient of one unique row, columns (cb + lane + k*G), into `acc` (zero on entry): its chunk sums when
@@ -550,7 +649,8 @@ __device__ __forceinline__ void row_gradient(const BwdParams& p, const RunMeta& 
     const int rs = m.rs, re = m.rs + m.len;
     const bool chunked = m.chunk_base >= 0;
     if (chunked) {
-        const int nc = chunks_of_run(m.len, p.chunk);
+        int nc = chunks_of_run(m.len, p.chunk);
+        if (p.long_chunks > 0 && nc > p.long_chunks) nc = 1;  // long_run_kernel left the total in the first slot
         int c = 0;
         for (; c + 4 <= nc; c += 4) {
             typename V::T v[4][K];
@@ -578,9 +678,9 @@ __device__ __forceinline__ void row_gradient(const BwdParams& p, const RunMeta& 
     } else if (first_direct) {
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = add4(acc[k], map4(g0[k], [&](float x) { return prep_grad(p, x, 1.0f); }));
-        if (re > rs + 1) sum_grad_rows<V, G, K>(p, rs + 1, re, cb, lane, nvec, acc);
+        if (re > rs + 1) sum_short_run<V, G, K>(p, rs + 1, re, cb, lane, nvec, acc);
     } else {
-        sum_grad_rows<V, G, K>(p, rs, re, cb, lane, nvec, acc);
+        sum_short_run<V, G, K>(p, rs, re, cb, lane, nvec, acc);
     }
 }
 
@@ -801,19 +901,12 @@ __global__ void __launch_bounds__(256) update_kernel(BwdParams p, const RunMeta*
             if (m.D & kMetaVecBit)
                 update_body<V4, G, K, OPT>(p, m, lane, D);
             else
-                update_body<V1, G, K, OPT>(p, m, lane, D);
+                update_body<V1, G, 4, OPT>(p, m, lane, D);  // word by word, four words per lane
         }
         lo = nlo;
         hi = nhi;
         r = rn;
     }
-}
-
-template <int G>
-__device__ __forceinline__ unsigned group_mask()
-{
-    if (G == 32) return kFullMask;
-    return ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
 }
 
 }  // namespace recsdk
