@@ -516,4 +516,254 @@ static inline int radix_sort_pairs_fused(const RadixFusedPlan& pl, KeyT* keys_a,
     return cur;
 }
 
+// ----------------------------------------------------------------------------
+// The same sort for large inputs, bound by memory instead of launches.  Per pass: tile histograms (keys read once,
+// counted in shared memory) -> per-digit scan across tiles -> scatter.  Tiles are 512 threads x kItems, and a tile's
+// pairs are put in digit order in shared memory first, so that they leave as runs of consecutive addresses: with 512
+// digits a tile of 2048 writes 4 pairs of 4 bytes to one place, a tile of 8192 sixteen, and a store instruction
+// of the reordered tile touches a few 128-byte lines instead of up to 32.  The histogram of a pass is not counted by
+// the producer of its input as in the fused mode above: one global atomic per pair and pass cost more than reading
+// the keys again.
+// 20 M pairs, 27-bit keys, beside the forward on another stream: 3 x (370 + 140) us in the fused mode, 3 x (157 + 43 + 8) us
+// here, and the kernel that writes the pairs 270 instead of 330 us.
+// ----------------------------------------------------------------------------
+constexpr int kBigThreads = 512;
+template <typename KeyT>
+__host__ __device__ constexpr int big_items()
+{
+    return sizeof(KeyT) == 4 ? 16 : 8;
+}
+static inline int64_t big_tiles(int64_t n, int items) { return ceil_div(n > 0 ? n : 1, static_cast<int64_t>(kBigThreads) * items); }
+static inline int64_t big_stride(int64_t tiles) { return ceil_div(tiles, 8) * 8; }  // histogram rows start on 32 bytes
+
+template <typename KeyT, int BITS>
+__global__ void __launch_bounds__(kBigThreads) big_hist_kernel(const KeyT* __restrict__ keys, int64_t n, int shift,
+                                                               uint32_t* __restrict__ hist, int64_t stride)
+{
+    constexpr int RADIX = 1 << BITS, ITEMS = big_items<KeyT>();
+    __shared__ uint32_t h[RADIX];
+    for (int d = threadIdx.x; d < RADIX; d += kBigThreads) h[d] = 0;
+    __syncthreads();
+    const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * (kBigThreads * ITEMS);
+    __align__(16) KeyT key[ITEMS];
+    if (tile0 + kBigThreads * ITEMS <= n) {
+        constexpr int VEC = 16 / sizeof(KeyT);
+#pragma unroll
+        for (int k = 0; k < ITEMS / VEC; ++k)
+            *reinterpret_cast<uint4*>(key + k * VEC) =
+                reinterpret_cast<const uint4*>(keys + tile0)[k * kBigThreads + threadIdx.x];
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) atomicAdd(&h[static_cast<unsigned>(key[k] >> shift) & (RADIX - 1)], 1u);
+    } else {
+        for (int64_t i = tile0 + threadIdx.x; i < n; i += kBigThreads)
+            atomicAdd(&h[static_cast<unsigned>(keys[i] >> shift) & (RADIX - 1)], 1u);
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < RADIX; d += kBigThreads) hist[d * stride + blockIdx.x] = h[d];
+}
+
+// One block per digit: exclusive scan of its row in place, eight tiles per thread and round; total -> totals[d].
+// Words of a row past its last tile are padding: read as they are, never used.
+static __global__ void __launch_bounds__(256) big_scan_kernel(uint32_t* __restrict__ hist, int64_t tiles, int64_t stride,
+                                                              uint32_t* __restrict__ totals)
+{
+    __shared__ int sm[33];
+    uint32_t* row = hist + blockIdx.x * stride;
+    uint32_t carry = 0;
+    for (int64_t base = 0; base < tiles; base += 256 * 8) {
+        const int64_t i = base + threadIdx.x * 8;
+        __align__(16) uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (i < tiles) {
+            *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(row + i);
+            *reinterpret_cast<uint4*>(v + 4) = *reinterpret_cast<const uint4*>(row + i + 4);
+        }
+        uint32_t s = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (i + k >= tiles) v[k] = 0;
+            s += v[k];
+        }
+        int total;
+        uint32_t run = carry + static_cast<uint32_t>(block_inclusive_scan(static_cast<int>(s), sm, &total)) - s;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t x = v[k];
+            v[k] = run;
+            run += x;
+        }
+        if (i < tiles) {
+            *reinterpret_cast<uint4*>(row + i) = *reinterpret_cast<const uint4*>(v);
+            *reinterpret_cast<uint4*>(row + i + 4) = *reinterpret_cast<const uint4*>(v + 4);
+        }
+        carry += static_cast<uint32_t>(total);
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+template <typename KeyT, int BITS>
+static inline size_t big_scatter_smem()
+{
+    constexpr size_t tile = static_cast<size_t>(kBigThreads) * big_items<KeyT>(), radix = size_t(1) << BITS;
+    return tile * (sizeof(KeyT) + sizeof(uint32_t)) + (kBigThreads / 32) * radix * sizeof(uint16_t) + radix * sizeof(uint32_t);
+}
+
+template <typename KeyT, int BITS>
+__global__ void __launch_bounds__(kBigThreads, 2) big_scatter_kernel(const KeyT* __restrict__ keys_in,
+                                                                     const uint32_t* __restrict__ vals_in,
+                                                                     KeyT* __restrict__ keys_out,
+                                                                     uint32_t* __restrict__ vals_out, int64_t n, int shift,
+                                                                     const uint32_t* __restrict__ hist,
+                                                                     const uint32_t* __restrict__ totals, int64_t stride)
+{
+    constexpr int RADIX = 1 << BITS, ITEMS = big_items<KeyT>(), WARPS = kBigThreads / 32, TILE = kBigThreads * ITEMS;
+    constexpr int PER = RADIX > kBigThreads ? RADIX / kBigThreads : 1;  // digits per thread in the block-wide steps
+    extern __shared__ __align__(16) unsigned char big_smem[];
+    __shared__ int sm[33];
+    KeyT* skey = reinterpret_cast<KeyT*>(big_smem);
+    uint32_t* sval = reinterpret_cast<uint32_t*>(skey + TILE);
+    uint32_t* gbase = sval + TILE;                                  // [RADIX] global position of local position 0
+    uint16_t* wcnt = reinterpret_cast<uint16_t*>(gbase + RADIX);   // [WARPS][RADIX]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int w = threadIdx.x; w < WARPS * RADIX / 2; w += kBigThreads) reinterpret_cast<uint32_t*>(wcnt)[w] = 0;
+
+    const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * TILE;
+    const int count = n - tile0 < TILE ? static_cast<int>(n - tile0) : TILE;
+    const int first = warp * (ITEMS * 32) + lane;  // a warp owns ITEMS * 32 consecutive pairs, taken 32 at a time
+    KeyT key[ITEMS];
+    uint16_t rank[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) key[r] = first + r * 32 < count ? keys_in[tile0 + first + r * 32] : KeyT(0);
+    uint32_t tot[PER], mine_hist[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int d = threadIdx.x * PER + q;
+        tot[q] = d < RADIX ? totals[d] : 0;
+        mine_hist[q] = d < RADIX ? hist[d * stride + blockIdx.x] : 0;
+    }
+    __syncthreads();
+    uint16_t* mine = wcnt + warp * RADIX;
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = first + r * 32 < count;
+        // lanes without a pair get a tag no other lane has
+        const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & (RADIX - 1) : RADIX + lane;
+        const unsigned peers = __match_any_sync(kFullMask, tag);
+        const unsigned before = __popc(peers & lanemask_lt());
+        const uint32_t prev = valid ? mine[tag] : 0;
+        __syncwarp();
+        if (valid && before == 0) mine[tag] = static_cast<uint16_t>(prev + __popc(peers));
+        __syncwarp();
+        rank[r] = static_cast<uint16_t>(prev + before);
+    }
+    __syncthreads();
+    {
+        // per digit: prefix over the warps, then where the digit starts in the tile and in the output
+        uint32_t cnt[PER];
+        int sum_tot = 0, sum_cnt = 0;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int d = threadIdx.x * PER + q;
+            uint32_t run = 0;
+            if (d < RADIX) {
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) {
+                    const uint32_t c = wcnt[w * RADIX + d];
+                    wcnt[w * RADIX + d] = static_cast<uint16_t>(run);
+                    run += c;
+                }
+            }
+            cnt[q] = run;
+            sum_cnt += static_cast<int>(run);
+            sum_tot += static_cast<int>(tot[q]);
+        }
+        int all;
+        uint32_t digit_base = static_cast<uint32_t>(block_inclusive_scan(sum_tot, sm, &all) - sum_tot);
+        uint32_t local = static_cast<uint32_t>(block_inclusive_scan(sum_cnt, sm, &all) - sum_cnt);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int d = threadIdx.x * PER + q;
+            if (d < RADIX) {
+                gbase[d] = digit_base + mine_hist[q] - local;  // wraps around; the sum with a local position does not
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) wcnt[w * RADIX + d] = static_cast<uint16_t>(wcnt[w * RADIX + d] + local);
+            }
+            digit_base += tot[q];
+            local += cnt[q];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        if (first + r * 32 < count) {
+            const unsigned d = static_cast<unsigned>(key[r] >> shift) & (RADIX - 1);
+            const int pos = mine[d] + rank[r];
+            skey[pos] = key[r];
+            sval[pos] = vals_in[tile0 + first + r * 32];
+        }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < count; i += kBigThreads) {
+        const KeyT k = skey[i];
+        const uint32_t pos = gbase[static_cast<unsigned>(k >> shift) & (RADIX - 1)] + static_cast<uint32_t>(i);
+        keys_out[pos] = k;
+        vals_out[pos] = sval[i];
+    }
+}
+
+template <typename KeyT, int BITS>
+static inline bool radix_sort_pass_big(const KeyT* kin, const uint32_t* vin, KeyT* kout, uint32_t* vout, int64_t n, int shift,
+                                       uint32_t* scratch, bool ready_only, cudaStream_t st)
+{
+    static bool optin_done[kMaxDevices] = {false};  // one table per instantiation
+    const size_t smem = big_scatter_smem<KeyT, BITS>();
+    if (!smem_optin(big_scatter_kernel<KeyT, BITS>, static_cast<int>(smem), optin_done)) return false;
+    if (ready_only) return true;
+    const int64_t tiles = big_tiles(n, big_items<KeyT>()), stride = big_stride(tiles);
+    uint32_t* hist = scratch;
+    uint32_t* totals = scratch + stride * (int64_t(1) << BITS);
+    const unsigned grid = static_cast<unsigned>(tiles);
+    big_hist_kernel<KeyT, BITS><<<grid, kBigThreads, 0, st>>>(kin, n, shift, hist, stride);
+    big_scan_kernel<<<1 << BITS, 256, 0, st>>>(hist, tiles, stride, totals);
+    big_scatter_kernel<KeyT, BITS><<<grid, kBigThreads, smem, st>>>(kin, vin, kout, vout, n, shift, hist, totals, stride);
+    return true;
+}
+
+// From this many pairs the three launches of a pass are worth it: 330 K pairs of 22 bits take 3 x 16.5 us this way and
+// 3 x 11.5 us by the fused mode, 1.7 M pairs 3 x 32.6 us and 3 x 52 us (both beside the forward).
+constexpr int64_t kSortBigN = int64_t(1) << 20;
+
+// Does an input of n pairs take the large path?  (Its scratch fits sort_scratch_u32_fused(n) words.)
+template <typename KeyT>
+static inline bool radix_sort_is_big(int64_t n, int key_bits)
+{
+    if (n < kSortBigN || key_bits <= 0) return false;
+    int passes, bits;
+    radix_plan(key_bits, &passes, &bits);
+    if (bits == 10) return radix_sort_pass_big<KeyT, 10>(nullptr, nullptr, nullptr, nullptr, n, 0, nullptr, true, nullptr);
+    if (bits == 9) return radix_sort_pass_big<KeyT, 9>(nullptr, nullptr, nullptr, nullptr, n, 0, nullptr, true, nullptr);
+    return radix_sort_pass_big<KeyT, 8>(nullptr, nullptr, nullptr, nullptr, n, 0, nullptr, true, nullptr);
+}
+
+// Same contract and same number of passes as radix_sort_pairs.
+template <typename KeyT>
+static inline int radix_sort_pairs_big(KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b, uint32_t* vals_b, int64_t n, int key_bits,
+                                       uint32_t* scratch, cudaStream_t st)
+{
+    int passes, bits;
+    radix_plan(key_bits, &passes, &bits);
+    int cur = 0;
+    for (int p = 0; p < passes; ++p) {
+        KeyT* kin = cur ? keys_b : keys_a;
+        uint32_t* vin = cur ? vals_b : vals_a;
+        KeyT* kout = cur ? keys_a : keys_b;
+        uint32_t* vout = cur ? vals_a : vals_b;
+        if (bits == 10) radix_sort_pass_big<KeyT, 10>(kin, vin, kout, vout, n, p * 10, scratch, false, st);
+        else if (bits == 9) radix_sort_pass_big<KeyT, 9>(kin, vin, kout, vout, n, p * 9, scratch, false, st);
+        else radix_sort_pass_big<KeyT, 8>(kin, vin, kout, vout, n, p * 8, scratch, false, st);
+        cur ^= 1;
+    }
+    return cur;
+}
+
 }  // namespace recsdk

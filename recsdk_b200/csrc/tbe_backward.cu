@@ -174,15 +174,18 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
         // The plan needs the indices and the LAYOUT of the gradient, not the gradient: it can run ahead, on
         // another stream, while the forward of the same batch (or the dense part) runs.
         cudaMemsetAsync(ws.counters, 0, 8 * sizeof(int64_t), st);  // {U, chunks, indices in chunked runs, unaligned columns, ...}
-        // 1. expand; it also fills the histogram of the first sort pass
-        const RadixFusedPlan plan = radix_fused_begin(N, key_bits, ws.sort_scratch, st);
+        // 1. expand; unless the sort is the one for large inputs it also fills the histogram of the first pass
+        const bool big = radix_sort_is_big<KeyT>(N, key_bits);
+        RadixFusedPlan plan{};
+        if (!big) plan = radix_fused_begin(N, key_bits, ws.sort_scratch, st);
         if (a->pooling_mode == RECSDK_POOL_NONE)
             expand_nobag_kernel<KeyT><<<grid_for(N, 256), 256, 0, st>>>(p, ka, ws.vals_a, plan.first, ws.counters);
         else
             expand_pooled_kernel<KeyT><<<grid_for(a->T * a->B, 8 * 32), 256, 0, st>>>(p, ka, ws.vals_a, plan.first,
                                                                                         ws.counters);
-        // 2. sort: per pass a scan and a scatter that fills the next pass's histogram
-        const int got = radix_sort_pairs_fused<KeyT>(plan, ka, ws.vals_a, kb, ws.vals_b, N, ws.sort_scratch, st);
+        // 2. sort: per pass a scan and a scatter that fills the next pass's histogram, or (large) three kernels
+        const int got = big ? radix_sort_pairs_big<KeyT>(ka, ws.vals_a, kb, ws.vals_b, N, key_bits, ws.sort_scratch, st)
+                            : radix_sort_pairs_fused<KeyT>(plan, ka, ws.vals_a, kb, ws.vals_b, N, ws.sort_scratch, st);
         if (got != which) return RECSDK_ERR_CUDA;  // cannot happen: both follow radix_plan
         // 3. runs
         device_scan_fn<true>(HeadFlagIn<KeyT>{keys}, RunStartOut{ws.run_start, ws.counters}, N, ws.scan_scratch,
