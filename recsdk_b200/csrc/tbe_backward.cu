@@ -148,6 +148,14 @@ static void launch_partial(const BwdParams& p, int64_t N, cudaStream_t st)
     } while (0)
 
 template <typename KeyT>
+static bool plan_small_ready(const recsdk_tbe_backward_args* a)
+{
+    static bool optin_done[kMaxDevices] = {false};  // one table per instantiation
+    return a->N <= kSmallN && a->T * a->B <= kSmallN &&
+           smem_optin(plan_small_kernel<KeyT>, static_cast<int>(plan_small_smem<KeyT>()), optin_done);
+}
+
+template <typename KeyT>
 static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const BwdWorkspace& ws, int key_bits,
                         cudaStream_t st)
 {
@@ -159,7 +167,8 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     // where the sorted tags end up depends only on the number of passes
     int passes, bits;
     radix_plan(key_bits, &passes, &bits);
-    const int which = (N > 1 ? passes : 0) & 1;
+    const bool small = plan_small_ready<KeyT>(a);  // leaves them in the a-buffer
+    const int which = small ? 0 : (N > 1 ? passes : 0) & 1;
     const KeyT* keys = which ? kb : ka;
     p.vals = which ? ws.vals_b : ws.vals_a;
     p.run_start = ws.run_start;
@@ -170,7 +179,10 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     p.long_chunks = (N >= kLongRunMinIds && p.chunk > 0) ? kLongChunks : 0;
     p.long_list = ws.long_list;
     const int vec_per_row = (a->max_D + 3) / 4;
-    if (do_plan) {
+    if (do_plan && small) {
+        plan_small_kernel<KeyT><<<1, kSmallThreads, plan_small_smem<KeyT>(), st>>>(p, key_bits, ws.vals_a, ws.run_start,
+                                                                                  ws.counters, ws.meta, ws.desc);
+    } else if (do_plan) {
         // The plan needs the indices and the LAYOUT of the gradient, not the gradient: it can run ahead, on
         // another stream, while the forward of the same batch (or the dense part) runs.
         cudaMemsetAsync(ws.counters, 0, 8 * sizeof(int64_t), st);  // {U, chunks, indices in chunked runs, unaligned columns, ...}

@@ -131,15 +131,60 @@ __device__ __forceinline__ int64_t feature_of_position(const int64_t* offs, int6
 // Features that share a table put gradient rows of different column offsets into ONE run, so the 128-bit path
 // is taken only when the column offset of EVERY feature is a multiple of four floats.  Block 0 of the expand
 // kernel checks that and raises counters[3] (zeroed before the plan) when one is not.
-__device__ __forceinline__ void flag_unaligned_columns(const BwdParams& p, int64_t* counters_rw)
+__device__ __forceinline__ bool unaligned_columns(const BwdParams& p)
 {
-    if (blockIdx.x != 0) return;
     bool bad = false;
     for (int64_t t = threadIdx.x; t < p.T; t += blockDim.x) {
         const int32_t c = p.sh.num_shards > 0 ? p.sh.col_offsets[t] : p.dofs[t];
         bad = bad || ((c | (p.dofs[t + 1] - p.dofs[t])) & 3) != 0;
     }
-    if (bad) atomicCAS(reinterpret_cast<unsigned long long*>(counters_rw + 3), 0ull, 1ull);
+    return bad;
+}
+__device__ __forceinline__ void flag_unaligned_columns(const BwdParams& p, int64_t* counters_rw)
+{
+    if (blockIdx.x != 0) return;
+    if (unaligned_columns(p)) atomicCAS(reinterpret_cast<unsigned long long*>(counters_rw + 3), 0ull, 1ull);
+}
+
+// key of the row that position `pos` of feature f takes
+__device__ __forceinline__ int64_t row_key(const BwdParams& p, int64_t f, int64_t pos)
+{
+    return p.uid != nullptr ? p.uinv[pos] + p.uoff[f] : p.cumsum[f] + p.idx[pos];
+}
+
+// The positions of the 32 bags from bag0 on, 32 at a time: emit(has a position, position, key, tag), called by all
+// lanes of the warp.
+template <typename Emit>
+__device__ __forceinline__ void expand_bags(const BwdParams& p, int64_t bag0, int lane, Emit emit)
+{
+    const int64_t num_bags = p.T * p.B;
+    const int64_t bag = bag0 + lane;
+    const int64_t start = bag < num_bags ? p.offs[bag] : INT64_MAX;  // lane l: first position of bag0+l
+    const int64_t last_bag = (bag0 + 32 < num_bags) ? bag0 + 32 : num_bags;
+    int64_t p0 = p.offs[bag0], p1 = p.offs[last_bag];
+    if (p0 < 0 || p1 > p.N || p0 > p1) {
+        // offsets that do not describe N positions (e.g. a buffer rewritten under a plan made ahead): never write
+        // past the workspace
+        set_status(p.status, RECSDK_ERR_INDEX_RANGE, p1, p.N);
+        p0 = p0 < 0 ? 0 : (p0 > p.N ? p.N : p0);
+        p1 = p1 > p.N ? p.N : (p1 < p0 ? p0 : p1);
+    }
+    const uint32_t f_l = bag < num_bags ? static_cast<uint32_t>(bag / p.B) : 0u;
+    const uint32_t b_l = bag < num_bags ? static_cast<uint32_t>(bag - static_cast<int64_t>(f_l) * p.B) : 0u;
+    for (int64_t base = p0; base < p1; base += 32) {
+        const int64_t pos = base + lane;
+        // largest j with start_j <= pos (bags with equal starts are empty; the last one owns pos)
+        int j = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+            const int cand = j + step;
+            const int64_t sc = __shfl_sync(kFullMask, start, cand & 31);
+            if (cand < 32 && sc <= pos) j = cand;
+        }
+        const uint32_t f = __shfl_sync(kFullMask, f_l, j);
+        const uint32_t b = __shfl_sync(kFullMask, b_l, j);
+        emit(pos < p1, pos, pos < p1 ? row_key(p, f, pos) : 0, (f << p.bshift) | b);
+    }
 }
 
 template <typename KeyT>
@@ -152,41 +197,14 @@ __global__ void __launch_bounds__(256) expand_pooled_kernel(BwdParams p, KeyT* _
     const int64_t num_bags = p.T * p.B;
     const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     for (int64_t bag0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * 32; bag0 < num_bags;
-         bag0 += warps_total * 32) {
-        const int64_t bag = bag0 + lane;
-        const int64_t start = bag < num_bags ? p.offs[bag] : INT64_MAX;  // lane l: first position of bag0+l
-        const int64_t last_bag = (bag0 + 32 < num_bags) ? bag0 + 32 : num_bags;
-        int64_t p0 = p.offs[bag0], p1 = p.offs[last_bag];
-        if (p0 < 0 || p1 > p.N || p0 > p1) {
-            // offsets that do not describe N positions (e.g. a buffer rewritten under a plan made ahead): never write
-            // past the workspace
-            set_status(p.status, RECSDK_ERR_INDEX_RANGE, p1, p.N);
-            p0 = p0 < 0 ? 0 : (p0 > p.N ? p.N : p0);
-            p1 = p1 > p.N ? p.N : (p1 < p0 ? p0 : p1);
-        }
-        const uint32_t f_l = bag < num_bags ? static_cast<uint32_t>(bag / p.B) : 0u;
-        const uint32_t b_l = bag < num_bags ? static_cast<uint32_t>(bag - static_cast<int64_t>(f_l) * p.B) : 0u;
-        for (int64_t base = p0; base < p1; base += 32) {
-            const int64_t pos = base + lane;
-            // largest j with start_j <= pos (bags with equal starts are empty; the last one owns pos)
-            int j = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const int cand = j + step;
-                const int64_t sc = __shfl_sync(kFullMask, start, cand & 31);
-                if (cand < 32 && sc <= pos) j = cand;
-            }
-            const uint32_t f = __shfl_sync(kFullMask, f_l, j);
-            const uint32_t b = __shfl_sync(kFullMask, b_l, j);
-            int64_t key = 0;
-            if (pos < p1) {
-                key = p.uid != nullptr ? p.uinv[pos] + p.uoff[f] : p.cumsum[f] + p.idx[pos];
+         bag0 += warps_total * 32)
+        expand_bags(p, bag0, lane, [&](bool have, int64_t pos, int64_t key, uint32_t tag) {
+            if (have) {
                 keys[pos] = static_cast<KeyT>(key);
-                vals[pos] = (f << p.bshift) | b;
+                vals[pos] = tag;
             }
-            sink.add_warp(pos < p1, static_cast<KeyT>(key), pos);
-        }
-    }
+            sink.add_warp(have, static_cast<KeyT>(key), pos);
+        });
 }
 
 template <typename KeyT>
@@ -201,8 +219,7 @@ __global__ void __launch_bounds__(256) expand_nobag_kernel(BwdParams p, KeyT* __
         const int64_t pos = pos0 + (threadIdx.x & 31);
         int64_t key = 0;
         if (pos < p.N) {
-            const int64_t f = feature_of_position(p.offs, p.T, p.B, pos);
-            key = p.uid != nullptr ? p.uinv[pos] + p.uoff[f] : p.cumsum[f] + p.idx[pos];
+            key = row_key(p, feature_of_position(p.offs, p.T, p.B, pos), pos);
             keys[pos] = static_cast<KeyT>(key);
             vals[pos] = static_cast<uint32_t>(pos);
         }
@@ -424,10 +441,9 @@ __device__ __forceinline__ void run_geometry(const BwdParams& p, uint32_t v0, in
 // 128-bit path for a run of feature f's table: needs every address the run touches 16-byte aligned, i.e. the
 // table (wofs, D), the row pitch of the gradient, and the column offsets of ALL features (counters[3], see
 // flag_unaligned_columns: a run can hold gradient rows of several features that share the table).
-__device__ __forceinline__ bool vec_ok_for(const BwdParams& p, int64_t wofs, int32_t D, int64_t f)
+__device__ __forceinline__ bool vec_ok_for(const BwdParams& p, int64_t wofs, int32_t D, bool unaligned_cols)
 {
-    (void)f;
-    if (!p.base_aligned || p.counters[3] != 0) return false;
+    if (!p.base_aligned || unaligned_cols) return false;
     if (p.sh.num_shards > 0) return ((wofs | D | p.sh.row_stride | p.max_D) & 3) == 0;
     return ((wofs | D | p.total_D | p.max_D) & 3) == 0;
 }
@@ -478,7 +494,7 @@ __global__ void __launch_bounds__(256, chunk_blocks(G)) partial_kernel(BwdParams
         const int2 be = p.chunk_desc[c];
         run_geometry(p, p.vals[be.x], D, wofs, f);
         float* out = p.partial + c * p.max_D;
-        if (vec_ok_for(p, wofs, D, f))
+        if (vec_ok_for(p, wofs, D, p.counters[3] != 0))
             partial_body<V4, G, K, chunk_loads(G) / K>(p, be, out, lane, D);
         else
             partial_body<V1, G, 4, 4>(p, be, out, lane, D);
@@ -548,6 +564,42 @@ constexpr int32_t kMetaVecBit = 1 << 30;
 // counter; slot numbers differ from launch to launch but a slot's content and the order in which
 // a run's slots are summed do not) and describes each chunk as [begin, end) in sorted positions.
 // counters[2] collects how many indices live in chunked runs (bandwidth accounting only).
+__device__ __forceinline__ RunMeta make_run_meta(const BwdParams& p, int64_t r, int rs, int re, int64_t key, uint32_t v0,
+                                                 bool unaligned_cols, int64_t* __restrict__ counters, int2* __restrict__ desc)
+{
+    const int len = re - rs;
+    int32_t D;
+    int64_t wofs, f;
+    run_geometry(p, v0, D, wofs, f);
+    const int64_t row = p.uid != nullptr ? p.uid[key] : key - p.cumsum[f];
+    RunMeta m;
+    m.row_off = wofs + row * D;
+    if (p.w_numel > 0 && (row < 0 || m.row_off + D > p.w_numel)) {
+        set_status(p.status, RECSDK_ERR_INDEX_RANGE, row, m.row_off);
+        m.row_off = -1;
+    }
+    m.g0_loc = grad_row_loc(p, v0);
+    m.rs = rs;
+    m.len = len;
+    m.D = D | (vec_ok_for(p, wofs, D, unaligned_cols) ? kMetaVecBit : 0);
+    m.chunk_base = -1;
+    if (len > p.direct_max) {
+        const int c = chunks_of_run(len, p.chunk);
+        const int step = p.chunk > 0 ? p.chunk : len;
+        const int base = static_cast<int>(atomicAdd(reinterpret_cast<unsigned long long*>(counters + 1),
+                                                    static_cast<unsigned long long>(c)));
+        atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), static_cast<unsigned long long>(len));
+        m.chunk_base = base;
+        if (p.long_chunks > 0 && c > p.long_chunks)
+            p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(counters + 4), 1ull)] = static_cast<int>(r);
+        for (int k = 0; k < c; ++k) {
+            const int b0 = rs + k * step;
+            desc[base + k] = make_int2(b0, b0 + step < re ? b0 + step : re);
+        }
+    }
+    return m;
+}
+
 template <typename KeyT>
 __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* __restrict__ keys,
                                                        int64_t* __restrict__ counters, RunMeta* __restrict__ meta,
@@ -557,43 +609,149 @@ __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* 
     for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < U;
          r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int rs = p.run_start[r], re = p.run_start[r + 1];
-        const int len = re - rs;
-        const int64_t key = static_cast<int64_t>(keys[rs]);
-        const uint32_t v0 = p.vals[rs];
-        int32_t D;
-        int64_t wofs, f;
-        run_geometry(p, v0, D, wofs, f);
-        const int64_t row = p.uid != nullptr ? p.uid[key] : key - p.cumsum[f];
-        RunMeta m;
-        m.row_off = wofs + row * D;
-        if (p.w_numel > 0 && (row < 0 || m.row_off + D > p.w_numel)) {
-            set_status(p.status, RECSDK_ERR_INDEX_RANGE, row, m.row_off);
-            m.row_off = -1;
-        }
-        m.g0_loc = grad_row_loc(p, v0);
-        m.rs = rs;
-        m.len = len;
-        m.D = D | (vec_ok_for(p, wofs, D, f) ? kMetaVecBit : 0);
-        m.chunk_base = -1;
-        if (len > p.direct_max) {
-            const int c = chunks_of_run(len, p.chunk);
-            const int step = p.chunk > 0 ? p.chunk : len;
-            const int base = static_cast<int>(atomicAdd(reinterpret_cast<unsigned long long*>(counters + 1),
-                                                        static_cast<unsigned long long>(c)));
-            atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), static_cast<unsigned long long>(len));
-            m.chunk_base = base;
-            if (p.long_chunks > 0 && c > p.long_chunks)
-                p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(counters + 4), 1ull)] = static_cast<int>(r);
-            for (int k = 0; k < c; ++k) {
-                const int b0 = rs + k * step;
-                desc[base + k] = make_int2(b0, b0 + step < re ? b0 + step : re);
-            }
-        }
-        meta[r] = m;
+        meta[r] = make_run_meta(p, r, rs, re, static_cast<int64_t>(keys[rs]), p.vals[rs], p.counters[3] != 0, counters, desc);
     }
 }
 
 #ifndef RECSDK_EMULATE
+// ---------------------------------------------------------------------------- 1.-4. the whole plan of a small batch
+// One block does what expand, the sort passes, the run scan and the records do for a batch that fits its shared memory
+// (at most kSmallN positions in at most kSmallN bags).  Such a batch is bound by launches and by the latency of each
+// kernel's first loads, not by work: 4096 ids of 20-bit keys took eleven launches, 37 us of kernels and the gaps between them, against 25 us
+// in this one launch (a training step of them 116 -> 93..102 us).  A radix pass is a rank inside the warps (32 consecutive positions a round), a prefix
+// over the warps per digit, and a move in shared memory: stable, like the passes of the large sorts.
+constexpr int kSmallN = 8192;
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallItems = kSmallN / kSmallThreads;
+constexpr int kSmallBits = 8;
+template <typename KeyT>
+constexpr size_t plan_small_smem()
+{
+    return kSmallN * (sizeof(KeyT) + sizeof(uint32_t)) + (kSmallN + 4) * sizeof(int) +
+           (kSmallThreads / 32) * (size_t(1) << kSmallBits) * sizeof(uint16_t);
+}
+
+template <typename KeyT>
+__global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, int key_bits, uint32_t* __restrict__ vals_out,
+                                                                   int* __restrict__ run_start, int64_t* counters,
+                                                                   RunMeta* __restrict__ meta, int2* __restrict__ desc)
+{
+    constexpr int RADIX = 1 << kSmallBits, WARPS = kSmallThreads / 32;
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    __shared__ int sm[33];
+    KeyT* skey = reinterpret_cast<KeyT*>(small_smem);
+    uint32_t* sval = reinterpret_cast<uint32_t*>(skey + kSmallN);
+    int* srun = reinterpret_cast<int*>(sval + kSmallN);
+    uint16_t* wcnt = reinterpret_cast<uint16_t*>(srun + kSmallN + 4);  // [WARPS][RADIX]
+    const int n = static_cast<int>(p.N);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        skey[i] = 0;
+        sval[i] = 0;
+    }
+    if (threadIdx.x < 8) counters[threadIdx.x] = 0;
+    const bool unaligned_cols = __syncthreads_or(unaligned_columns(p) ? 1 : 0) != 0;
+    if (threadIdx.x == 0 && unaligned_cols) counters[3] = 1;
+    if (p.mode == RECSDK_POOL_NONE) {
+        for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+            skey[i] = static_cast<KeyT>(row_key(p, feature_of_position(p.offs, p.T, p.B, i), i));
+            sval[i] = static_cast<uint32_t>(i);
+        }
+    } else {
+        const int64_t num_bags = p.T * p.B;
+        for (int64_t bag0 = warp * 32; bag0 < num_bags; bag0 += WARPS * 32)
+            expand_bags(p, bag0, lane, [&](bool have, int64_t pos, int64_t key, uint32_t tag) {
+                if (have) {
+                    skey[pos] = static_cast<KeyT>(key);
+                    sval[pos] = tag;
+                }
+            });
+    }
+    __syncthreads();
+    const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
+    const int first = warp * rounds * 32 + lane;
+    uint16_t* mine = wcnt + warp * RADIX;
+    for (int shift = 0; shift < key_bits; shift += kSmallBits) {
+        KeyT key[kSmallItems];
+        uint32_t val[kSmallItems];
+        int rank[kSmallItems];
+        for (int w = threadIdx.x; w < WARPS * RADIX / 2; w += kSmallThreads) reinterpret_cast<uint32_t*>(wcnt)[w] = 0;
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r)
+            if (r < rounds && first + r * 32 < n) {
+                key[r] = skey[first + r * 32];
+                val[r] = sval[first + r * 32];
+            }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r)
+            if (r < rounds) {
+                const bool valid = first + r * 32 < n;
+                const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & (RADIX - 1) : RADIX + lane;
+                const unsigned peers = __match_any_sync(kFullMask, tag);
+                const unsigned before = __popc(peers & lanemask_lt());
+                const uint32_t prev = valid ? mine[tag] : 0;
+                __syncwarp();
+                if (valid && before == 0) mine[tag] = static_cast<uint16_t>(prev + __popc(peers));
+                __syncwarp();
+                rank[r] = static_cast<int>(prev + before);
+            }
+        __syncthreads();
+        int count = 0;
+        if (threadIdx.x < RADIX) {
+#pragma unroll 8
+            for (int w = 0; w < WARPS; ++w) {
+                const int c = wcnt[w * RADIX + threadIdx.x];
+                wcnt[w * RADIX + threadIdx.x] = static_cast<uint16_t>(count);
+                count += c;
+            }
+        }
+        int all;
+        const int base = block_inclusive_scan(count, sm, &all) - count;
+        if (threadIdx.x < RADIX) srun[threadIdx.x] = base;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r)
+            if (r < rounds && first + r * 32 < n) {
+                const unsigned d = static_cast<unsigned>(key[r] >> shift) & (RADIX - 1);
+                const int pos = srun[d] + mine[d] + rank[r];
+                skey[pos] = key[r];
+                sval[pos] = val[r];
+            }
+        __syncthreads();
+    }
+    // run starts: each thread looks at `rounds` consecutive positions
+    {
+        const int i0 = threadIdx.x * rounds;
+        int heads = 0;
+        for (int k = 0; k < rounds; ++k) {
+            const int i = i0 + k;
+            if (i < n) heads += (i == 0 || skey[i] != skey[i - 1]) ? 1 : 0;
+        }
+        int total;
+        int at = block_inclusive_scan(heads, sm, &total) - heads;
+        for (int k = 0; k < rounds; ++k) {
+            const int i = i0 + k;
+            if (i < n && (i == 0 || skey[i] != skey[i - 1])) {
+                srun[at] = i;
+                run_start[at] = i;
+                ++at;
+            }
+        }
+        if (threadIdx.x == 0) {
+            srun[total] = n;
+            run_start[total] = n;
+            counters[0] = total;
+        }
+        for (int i = threadIdx.x; i < n; i += kSmallThreads) vals_out[i] = sval[i];
+        __syncthreads();
+        for (int r = threadIdx.x; r < total; r += kSmallThreads) {
+            const int rs = srun[r];
+            meta[r] = make_run_meta(p, r, rs, srun[r + 1], static_cast<int64_t>(skey[rs]), sval[rs], unaligned_cols, counters,
+                                    desc);
+        }
+    }
+}
 // ---------------------------------------------------------------------------- 4c. totals of the longest runs
 // One warp per (listed run, 32 columns): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
 // place of the run's first chunk sum (no other warp reads these columns of this run).  The chunk sums come through a
