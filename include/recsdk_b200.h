@@ -313,6 +313,17 @@ RECSDK_API int recsdk_mapper_unique_out(const recsdk_mapper_t* m, const int64_t*
                                         int64_t* unique_inverse, int64_t* unique_offset, int64_t table_id,
                                         int64_t* dev_status, void* workspace, size_t workspace_bytes,
                                         void* stream);
+/* The same for tables first_table .. first_table + num_tables - 1 together, table i's segment being
+ * [seg_offsets[i], seg_offsets[i + 1]) (host array): a few launches for all of them.  workspaces[i] /
+ * workspace_bytes[i] as for the segment alone; mappers or workspaces that come up twice are taken one after the
+ * other.  dev_status: num_tables pointers or NULL; status_out (device, may be NULL): the status words of table t end
+ * up at [t * RECSDK_STATUS_WORDS], so that one read tells whether any table failed. */
+RECSDK_API int recsdk_mapper_unique_out_multi(const recsdk_mapper_t* const* mappers, int64_t num_tables,
+                                              int64_t first_table, const int64_t* ids, int64_t* hash_indices,
+                                              const int64_t* seg_offsets, int64_t* unique, int64_t* unique_ids,
+                                              int64_t* unique_inverse, int64_t* unique_offset,
+                                              int64_t* const* dev_status, int64_t* status_out, void* const* workspaces,
+                                              const size_t* workspace_bytes, void* stream);
 /* ids2indices_unique: slots for all ids (written to hash_indices), then SORTED
  * unique of the slots + inverse.  Workspace: max(mapper, unique_sorted). */
 RECSDK_API int recsdk_mapper_ids2indices_unique(const recsdk_mapper_t* m, const int64_t* ids, int64_t n,

@@ -146,6 +146,9 @@ SIGNATURES = {
     "recsdk_mapper_workspace_bytes": (C.c_size_t, [C.c_int64]),
     "recsdk_mapper_unique_out": (C.c_int, [C.POINTER(MapperT), vp, vp, C.c_int64, C.c_int64, vp, vp, vp, vp,
                                            C.c_int64, vp, vp, C.c_size_t, vp]),
+    "recsdk_mapper_unique_out_multi": (C.c_int, [C.POINTER(C.POINTER(MapperT)), C.c_int64, C.c_int64, vp, vp,
+                                                 C.POINTER(C.c_int64), vp, vp, vp, vp, C.POINTER(vp), vp, C.POINTER(vp),
+                                                 C.POINTER(C.c_size_t), vp]),
     "recsdk_mapper_ids2indices_unique": (C.c_int, [C.POINTER(MapperT), vp, C.c_int64, vp, vp, vp, vp, vp, vp,
                                                    C.c_size_t, vp]),
     "recsdk_swap_init": (C.c_int, [C.POINTER(SwapT), vp]),

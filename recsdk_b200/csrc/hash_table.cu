@@ -149,13 +149,10 @@ static bool is_pow2(int64_t x) { return x > 0 && (x & (x - 1)) == 0; }
 // and bids for it with its position; ent[i] = the entry, or -1 when the table is full.
 // MODE 0: mapper (negative key is an error), MODE 1: swap (-1 = not admitted -> slot 0).
 template <int MODE>
-static __global__ void __launch_bounds__(256) phase_find_or_claim_kernel(int64_t* __restrict__ table, int64_t cap,
-                                                                         const int64_t* __restrict__ keys, int64_t n,
-                                                                         int64_t* __restrict__ out_slots,
-                                                                         int64_t* __restrict__ ent, int* __restrict__ miss,
-                                                                         int64_t* __restrict__ slot_version,
-                                                                         const int64_t* __restrict__ counters,
-                                                                         int64_t* __restrict__ status)
+__device__ __forceinline__ void find_or_claim(int64_t* __restrict__ table, int64_t cap, const int64_t* __restrict__ keys,
+                                              int64_t n, int64_t* __restrict__ out_slots, int64_t* __restrict__ ent,
+                                              int* __restrict__ miss, int64_t* __restrict__ slot_version,
+                                              const int64_t* __restrict__ counters, int64_t* __restrict__ status)
 {
     const int64_t now = MODE == 1 ? counters[1] : 0;
     const int gl = threadIdx.x & (kProbeLanes - 1);
@@ -194,6 +191,18 @@ static __global__ void __launch_bounds__(256) phase_find_or_claim_kernel(int64_t
         ent[i] = e;
         miss[i] = 1;
     }
+}
+
+template <int MODE>
+static __global__ void __launch_bounds__(256) phase_find_or_claim_kernel(int64_t* __restrict__ table, int64_t cap,
+                                                                         const int64_t* __restrict__ keys, int64_t n,
+                                                                         int64_t* __restrict__ out_slots,
+                                                                         int64_t* __restrict__ ent, int* __restrict__ miss,
+                                                                         int64_t* __restrict__ slot_version,
+                                                                         const int64_t* __restrict__ counters,
+                                                                         int64_t* __restrict__ status)
+{
+    find_or_claim<MODE>(table, cap, keys, n, out_slots, ent, miss, slot_version, counters, status);
 }
 
 // phase 2, as the input of a scan: 1 where position i won the bid for its key.  The scan's consumer may overwrite
@@ -281,11 +290,9 @@ struct MapperAssignOut {
 // number of new keys (tmp[0], the scan's total); BID: every position also bids for its slot with its position
 // (first phase of the first-occurrence unique below).
 template <bool BID>
-static __global__ void __launch_bounds__(256) mapper_readback_kernel(recsdk_mapper_t m, int64_t n,
-                                                                     const int64_t* __restrict__ ent,
-                                                                     const int* __restrict__ miss,
-                                                                     int64_t* __restrict__ out_slots,
-                                                                     const int64_t* __restrict__ tmp)
+__device__ __forceinline__ void mapper_readback(const recsdk_mapper_t& m, int64_t n, const int64_t* __restrict__ ent,
+                                                const int* __restrict__ miss, int64_t* __restrict__ out_slots,
+                                                const int64_t* __restrict__ tmp)
 {
     RECSDK_GRID_STRIDE(i, n)
     {
@@ -308,8 +315,17 @@ static __global__ void __launch_bounds__(256) mapper_readback_kernel(recsdk_mapp
     }
 }
 
+static __global__ void __launch_bounds__(256) mapper_readback_kernel(recsdk_mapper_t m, int64_t n,
+                                                                     const int64_t* __restrict__ ent,
+                                                                     const int* __restrict__ miss,
+                                                                     int64_t* __restrict__ out_slots,
+                                                                     const int64_t* __restrict__ tmp)
+{
+    mapper_readback<false>(m, n, ent, miss, out_slots, tmp);
+}
+
 // first-occurrence unique of the slots of one segment (ids_mapper.cpp:115-174): the positions bid for their slot in
-// mapper_readback_kernel<true>; position i is a first occurrence when it holds the mark of its slot
+// mapper_readback<true>; position i is a first occurrence when it holds the mark of its slot
 struct HoldsMarkIn {
     const int64_t* slots;
     const int32_t* mark;
@@ -320,17 +336,11 @@ struct HoldsMarkIn {
         return (s >= 0 && s < max_index && mark[s] == static_cast<int>(i)) ? 1 : 0;
     }
 };
-static __global__ void __launch_bounds__(256) uniq_write_kernel(const int64_t* __restrict__ slots, int64_t n,
-                                                                const int32_t* __restrict__ mark, int64_t max_index,
-                                                                const int* __restrict__ rank,
-                                                                const int64_t* __restrict__ slot_key,
-                                                                int64_t* __restrict__ unique,
-                                                                int64_t* __restrict__ unique_ids,
-                                                                int64_t* __restrict__ inverse,
-                                                                int64_t* __restrict__ unique_offset, int64_t table_id,
-                                                                const int64_t* __restrict__ tmp)
+__device__ __forceinline__ void uniq_write(const int64_t* __restrict__ slots, int64_t n, const int32_t* __restrict__ mark,
+                                           int64_t max_index, const int* __restrict__ rank,
+                                           const int64_t* __restrict__ slot_key, int64_t* __restrict__ unique,
+                                           int64_t* __restrict__ unique_ids, int64_t* __restrict__ inverse, int64_t base)
 {
-    const int64_t base = table_id == 0 ? 0 : unique_offset[table_id];
     RECSDK_GRID_STRIDE(i, n)
     {
         const int64_t s = slots[i];
@@ -345,13 +355,9 @@ static __global__ void __launch_bounds__(256) uniq_write_kernel(const int64_t* _
         }
         inverse[i] = rank[holder];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (table_id == 0) unique_offset[0] = 0;
-        unique_offset[table_id + 1] = base + tmp[1];
-    }
 }
-static __global__ void __launch_bounds__(256) uniq_reset_kernel(const int64_t* __restrict__ slots, int64_t n,
-                                                                int32_t* __restrict__ mark, int64_t max_index)
+__device__ __forceinline__ void uniq_reset(const int64_t* __restrict__ slots, int64_t n, int32_t* __restrict__ mark,
+                                           int64_t max_index)
 {
     RECSDK_GRID_STRIDE(i, n)
     {
@@ -359,26 +365,177 @@ static __global__ void __launch_bounds__(256) uniq_reset_kernel(const int64_t* _
         if (s >= 0 && s < max_index) mark[s] = kMarkFree;
     }
 }
+
+// ---- several mappers at once ------------------------------------------------
+// The same phases over up to kMapperGroup tables, blockIdx.y = table: a hash-keyed module maps its keys table by table,
+// and one table's segment is a few ten thousand keys, so that each phase of each table is a launch-bound kernel on a
+// nearly empty chip.  8 tables of 33 K keys: 64 launches with 272 us in their kernels became 8
+// launches, and a training step on them went from 725 to 371 us (eight reads of a status word became one as well).
+struct MapperSeg {
+    recsdk_mapper_t m;
+    const int64_t* ids;
+    int64_t *slots, *inverse, *status;
+    int64_t* ent;
+    int *miss, *rank, *tiles_new, *tiles_uniq;
+    int64_t* totals;  // {new keys, unique slots}
+    int64_t n, table_id;
+};
+constexpr int kMapperGroup = 16;
+struct MapperGroup {
+    MapperSeg seg[kMapperGroup];
+};
+
+static __global__ void __launch_bounds__(256) group_find_or_claim_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    find_or_claim<0>(s.m.table, s.m.hash_capacity, s.ids, s.n, s.slots, s.ent, s.miss, nullptr, s.m.counters, s.status);
+}
+// Scan over one table's flags; tiles past the end of a short table have nothing to do.  The apply kernel adds up the
+// sums of the tiles before its own.
+template <typename InFn>
+__device__ __forceinline__ void group_scan_reduce(const InFn& in, int64_t n, int* tile_sums)
+{
+    __shared__ int sm[33];
+    if (static_cast<int64_t>(blockIdx.x) * kScanTile >= n) return;  // block-uniform
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanItems;
+    int s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+        if (base + k < n) s += in(base + k);
+    int total;
+    block_inclusive_scan(s, sm, &total);
+    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+}
+template <typename InFn, typename OutFn>
+__device__ __forceinline__ void group_scan_apply(const InFn& in, const OutFn& out, int64_t n, const int* tile_sums,
+                                                 int64_t* total_out)
+{
+    __shared__ int sm[33];
+    if (static_cast<int64_t>(blockIdx.x) * kScanTile >= n) {
+        if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) *total_out = 0;
+        return;
+    }
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanItems;
+    int v[kScanItems];
+    int s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        v[k] = (base + k < n) ? in(base + k) : 0;
+        s += v[k];
+    }
+    int total;
+    const int inc = block_inclusive_scan(s, sm, &total);
+    int part = 0, before;
+    for (int t = threadIdx.x; t < static_cast<int>(blockIdx.x); t += blockDim.x) part += tile_sums[t];
+    block_inclusive_scan(part, sm, &before);
+    int run = before + inc - s;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        if (base + k < n) out(base + k, v[k], run, n);
+        run += v[k];
+    }
+    if (base < n && base + kScanItems >= n) *total_out = run;  // the thread that holds the last item
+}
+static __global__ void __launch_bounds__(kScanThreads) group_new_reduce_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    group_scan_reduce(WonBidIn{s.m.table, s.ent, s.miss}, s.n, s.tiles_new);
+}
+static __global__ void __launch_bounds__(kScanThreads) group_new_assign_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    group_scan_apply(WonBidIn{s.m.table, s.ent, s.miss}, MapperAssignOut{s.m, s.ids, s.ent, s.status}, s.n, s.tiles_new,
+                     s.totals);
+}
+static __global__ void __launch_bounds__(256) group_readback_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    if (s.n > 0) mapper_readback<true>(s.m, s.n, s.ent, s.miss, s.slots, s.totals);
+}
+struct RankOut {
+    int* rank;
+    __device__ __forceinline__ void operator()(int64_t i, int, int prefix, int64_t) const { rank[i] = prefix; }
+};
+static __global__ void __launch_bounds__(kScanThreads) group_uniq_reduce_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    group_scan_reduce(HoldsMarkIn{s.slots, s.m.mark, s.m.init_max_index}, s.n, s.tiles_uniq);
+}
+static __global__ void __launch_bounds__(kScanThreads) group_uniq_rank_kernel(const __grid_constant__ MapperGroup g)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    group_scan_apply(HoldsMarkIn{s.slots, s.m.mark, s.m.init_max_index}, RankOut{s.rank}, s.n, s.tiles_uniq, s.totals + 1);
+}
+// a table's unique slots start where those of the tables before it end
+static __global__ void __launch_bounds__(256) group_uniq_write_kernel(const __grid_constant__ MapperGroup g,
+                                                                      int64_t* __restrict__ unique,
+                                                                      int64_t* __restrict__ unique_ids,
+                                                                      int64_t* __restrict__ unique_offset)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    const int64_t first = g.seg[0].table_id;
+    int64_t base = first == 0 ? 0 : unique_offset[first];
+    for (unsigned t = 0; t < blockIdx.y; ++t) base += g.seg[t].totals[1];
+    uniq_write(s.slots, s.n, s.m.mark, s.m.init_max_index, s.rank, s.m.slot_key, unique, unique_ids, s.inverse, base);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (s.table_id == 0) unique_offset[0] = 0;
+        unique_offset[s.table_id + 1] = base + s.totals[1];
+    }
+}
+// the marks are free again; `status_out` (optional) collects the status words of all tables, one read for the host
+static __global__ void __launch_bounds__(256) group_uniq_reset_kernel(const __grid_constant__ MapperGroup g,
+                                                                      int64_t* __restrict__ status_out)
+{
+    const MapperSeg& s = g.seg[blockIdx.y];
+    uniq_reset(s.slots, s.n, s.m.mark, s.m.init_max_index);
+    if (status_out != nullptr && blockIdx.x == 0 && threadIdx.x < RECSDK_STATUS_WORDS)
+        status_out[s.table_id * RECSDK_STATUS_WORDS + threadIdx.x] = s.status != nullptr ? s.status[threadIdx.x] : 0;
+}
+
 static __global__ void empty_segment_kernel(int64_t* unique_offset, int64_t table_id)
 {
     // ids_mapper.cpp:78-81
     unique_offset[table_id + 1] = unique_offset[table_id];
 }
+static __global__ void status_copy_kernel(const __grid_constant__ MapperGroup g, int tables, int64_t* __restrict__ status_out)
+{
+    for (int i = threadIdx.x; i < tables * RECSDK_STATUS_WORDS; i += blockDim.x) {
+        const MapperSeg& s = g.seg[i / RECSDK_STATUS_WORDS];
+        status_out[s.table_id * RECSDK_STATUS_WORDS + i % RECSDK_STATUS_WORDS] =
+            s.status != nullptr ? s.status[i % RECSDK_STATUS_WORDS] : 0;
+    }
+}
+
+static int mapper_group_run(const MapperGroup& g, int tables, int64_t max_n, int64_t* unique, int64_t* unique_ids,
+                            int64_t* unique_offset, int64_t* status_out, cudaStream_t st)
+{
+    const unsigned y = static_cast<unsigned>(tables);
+    const int64_t n = max_n > 0 ? max_n : 1;
+    const dim3 probe(static_cast<unsigned>(grid_for(n, 256 / kProbeLanes)), y), flat(static_cast<unsigned>(grid_for(n, 256)), y),
+        tiles(static_cast<unsigned>(scan_num_tiles(n)), y);
+    group_find_or_claim_kernel<<<probe, 256, 0, st>>>(g);
+    group_new_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    group_new_assign_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    group_readback_kernel<<<flat, 256, 0, st>>>(g);
+    group_uniq_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    group_uniq_rank_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    group_uniq_write_kernel<<<flat, 256, 0, st>>>(g, unique, unique_ids, unique_offset);
+    group_uniq_reset_kernel<<<flat, 256, 0, st>>>(g, status_out);
+    RECSDK_CUDA_CHECK_LAUNCH();
+    return RECSDK_OK;
+}
 
 // key -> slot for ids[0..n) (find or insert, first-come numbering): find-or-claim, a scan over "won the bid" whose
-// consumer numbers the new keys, read back.  `bid_marks`: the read-back also opens the first-occurrence unique.
+// consumer numbers the new keys, read back.
 static int mapper_map(const recsdk_mapper_t* m, const int64_t* ids, int64_t n, int64_t* hash_indices,
-                      int64_t* status, const MapperWs& ws, cudaStream_t st, bool bid_marks = false)
+                      int64_t* status, const MapperWs& ws, cudaStream_t st)
 {
     const int grid = grid_for(n, 256);
     phase_find_or_claim_kernel<0><<<grid_for(n, 256 / kProbeLanes), 256, 0, st>>>(
         m->table, m->hash_capacity, ids, n, hash_indices, ws.ent, ws.miss, nullptr, m->counters, status);
     device_scan_fn<false>(WonBidIn{m->table, ws.ent, ws.miss}, MapperAssignOut{*m, ids, ws.ent, status}, n,
                           ws.scan_scratch, ws.tmp, st);
-    if (bid_marks)
-        mapper_readback_kernel<true><<<grid, 256, 0, st>>>(*m, n, ws.ent, ws.miss, hash_indices, ws.tmp);
-    else
-        mapper_readback_kernel<false><<<grid, 256, 0, st>>>(*m, n, ws.ent, ws.miss, hash_indices, ws.tmp);
+    mapper_readback_kernel<<<grid, 256, 0, st>>>(*m, n, ws.ent, ws.miss, hash_indices, ws.tmp);
     RECSDK_CUDA_CHECK_LAUNCH();
     return RECSDK_OK;
 }
@@ -914,35 +1071,79 @@ extern "C" size_t recsdk_mapper_workspace_bytes(int64_t n)
     return a + b;
 }
 
+extern "C" int recsdk_mapper_unique_out_multi(const recsdk_mapper_t* const* mappers, int64_t num_tables, int64_t first_table,
+                                              const int64_t* ids, int64_t* hash_indices, const int64_t* seg_offsets,
+                                              int64_t* unique, int64_t* unique_ids, int64_t* unique_inverse,
+                                              int64_t* unique_offset, int64_t* const* dev_status, int64_t* status_out,
+                                              void* const* workspaces, const size_t* workspace_bytes, void* stream)
+{
+    if (!mappers || !seg_offsets || !unique_offset || !workspaces || !workspace_bytes || num_tables < 0 || first_table < 0)
+        return RECSDK_ERR_INVALID_ARG;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    for (int64_t t = 0; t < num_tables; ++t) {
+        const int64_t start = seg_offsets[t], n = seg_offsets[t + 1] - start;
+        if (!mappers[t] || start < 0 || n < 0) return RECSDK_ERR_INVALID_ARG;
+        if (n >= kMarkFree) return RECSDK_ERR_TOO_LARGE;
+        if (n > 0 && (!ids || !hash_indices || !unique || !unique_ids || !unique_inverse)) return RECSDK_ERR_INVALID_ARG;
+        if (n > 0 && (!workspaces[t] || carve_mapper(workspaces[t], n).bytes > workspace_bytes[t])) return RECSDK_ERR_WORKSPACE;
+    }
+    int64_t t = 0;
+    while (t < num_tables) {
+        // a group ends where a table or a workspace comes up again: those must not run side by side
+        MapperGroup g;
+        int k = 0;
+        int64_t max_n = 0;
+        for (; t < num_tables && k < kMapperGroup; ++t, ++k) {
+            const int64_t start = seg_offsets[t], n = seg_offsets[t + 1] - start;
+            bool again = false;
+            for (int j = 0; j < k; ++j)
+                again = again || g.seg[j].m.table == mappers[t]->table ||
+                        (n > 0 && g.seg[j].n > 0 && workspaces[t] == workspaces[t - k + j]);
+            if (again) break;
+            MapperSeg& s = g.seg[k];
+            s.m = *mappers[t];
+            s.n = n;
+            s.table_id = first_table + t;
+            s.ids = n > 0 ? ids + start : nullptr;
+            s.slots = n > 0 ? hash_indices + start : nullptr;
+            s.inverse = n > 0 ? unique_inverse + start : nullptr;
+            s.status = dev_status ? dev_status[t] : nullptr;
+            const MapperWs ws = carve_mapper(n > 0 ? workspaces[t] : nullptr, n);
+            s.ent = ws.ent;
+            s.miss = ws.miss;
+            s.rank = ws.rank;
+            s.tiles_new = ws.scan_scratch;
+            s.tiles_uniq = ws.first;  // at most one word per kScanTile positions
+            s.totals = ws.tmp;
+            max_n = n > max_n ? n : max_n;
+        }
+        // an empty segment may come without a workspace: its totals stand beside those of a neighbour that has one
+        int64_t* spare = nullptr;
+        for (int j = 0; j < k; ++j)
+            if (g.seg[j].n > 0) spare = g.seg[j].totals + 2;
+        if (max_n == 0) {
+            for (int j = 0; j < k; ++j) empty_segment_kernel<<<1, 1, 0, st>>>(unique_offset, g.seg[j].table_id);
+            if (status_out != nullptr) status_copy_kernel<<<1, 32, 0, st>>>(g, k, status_out);
+            continue;
+        }
+        for (int j = 0; j < k; ++j)
+            if (g.seg[j].n == 0) g.seg[j].totals = spare;
+        const int rc = mapper_group_run(g, k, max_n, unique, unique_ids, unique_offset, status_out, st);
+        if (rc != RECSDK_OK) return rc;
+    }
+    RECSDK_CUDA_CHECK_LAUNCH();
+    return RECSDK_OK;
+}
+
 extern "C" int recsdk_mapper_unique_out(const recsdk_mapper_t* m, const int64_t* ids, int64_t* hash_indices,
                                         int64_t seg_start, int64_t seg_len, int64_t* unique, int64_t* unique_ids,
                                         int64_t* unique_inverse, int64_t* unique_offset, int64_t table_id,
                                         int64_t* dev_status, void* workspace, size_t workspace_bytes, void* stream)
 {
     if (!m || seg_start < 0 || seg_len < 0 || table_id < 0 || !unique_offset) return RECSDK_ERR_INVALID_ARG;
-    if (seg_len >= kMarkFree) return RECSDK_ERR_TOO_LARGE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (seg_len == 0) {
-        empty_segment_kernel<<<1, 1, 0, st>>>(unique_offset, table_id);
-        RECSDK_CUDA_CHECK_LAUNCH();
-        return RECSDK_OK;
-    }
-    if (!ids || !hash_indices || !unique || !unique_ids || !unique_inverse) return RECSDK_ERR_INVALID_ARG;
-    if (!workspace) return RECSDK_ERR_WORKSPACE;
-    const MapperWs ws = carve_mapper(workspace, seg_len);
-    if (ws.bytes > workspace_bytes) return RECSDK_ERR_WORKSPACE;
-    const int64_t* seg_ids = ids + seg_start;
-    int64_t* seg_hi = hash_indices + seg_start;
-    int rc = mapper_map(m, seg_ids, seg_len, seg_hi, dev_status, ws, st, true);
-    if (rc != RECSDK_OK) return rc;
-    const int grid = grid_for(seg_len, 256);
-    device_scan_fn<false>(HoldsMarkIn{seg_hi, m->mark, m->init_max_index}, FlagRankOut{ws.first, ws.rank}, seg_len,
-                          ws.scan_scratch, ws.tmp + 1, st);
-    uniq_write_kernel<<<grid, 256, 0, st>>>(seg_hi, seg_len, m->mark, m->init_max_index, ws.rank, m->slot_key, unique,
-                                            unique_ids, unique_inverse + seg_start, unique_offset, table_id, ws.tmp);
-    uniq_reset_kernel<<<grid, 256, 0, st>>>(seg_hi, seg_len, m->mark, m->init_max_index);
-    RECSDK_CUDA_CHECK_LAUNCH();
-    return RECSDK_OK;
+    const int64_t seg[2] = {seg_start, seg_start + seg_len};
+    return recsdk_mapper_unique_out_multi(&m, 1, table_id, ids, hash_indices, seg, unique, unique_ids, unique_inverse,
+                                          unique_offset, &dev_status, nullptr, &workspace, &workspace_bytes, stream);
 }
 
 extern "C" int recsdk_mapper_ids2indices_unique(const recsdk_mapper_t* m, const int64_t* ids, int64_t n,

@@ -466,10 +466,9 @@ static void define_and_implement(torch::Library& m)
 }
 
 // ---------------------------------------------------------------------------- IdsMapper / bucketize
-static void raise_on_status(const Tensor& status, const char* where)
+// `s`: the status words, read back from `status`
+static void raise_on_status_words(const int64_t* s, const Tensor& status, const char* where)
 {
-    const Tensor h = status.cpu();  // synchronises, like the reference's TORCH_CHECK inside its host loop
-    const int64_t* s = h.data_ptr<int64_t>();
     if (s[0] == 0) return;
     const int code = static_cast<int>(s[0]);
     const int64_t d0 = s[1];
@@ -478,6 +477,11 @@ static void raise_on_status(const Tensor& status, const char* where)
     if (code == RECSDK_ERR_TABLE_FULL)
         TORCH_CHECK(false, where, ": Ids map reached maxIndex = ", d0, " please reallocate a larger buffer.");
     TORCH_CHECK(false, where, ": ", recsdk_error_string(code));
+}
+static void raise_on_status(const Tensor& status, const char* where)
+{
+    const Tensor h = status.cpu();  // synchronises, like the reference's TORCH_CHECK inside its host loop
+    raise_on_status_words(h.data_ptr<int64_t>(), status, where);
 }
 
 // NS tags the registration namespace (a C++ type can back only one registered class): 0 = recsdk::, 1 = hybrid::
@@ -523,7 +527,8 @@ public:
     void UniqueAndLookupOut(const Tensor& globalIds, const Tensor& hashIndices, const Tensor& offset, const Tensor& unique,
                             const Tensor& uniqueIds, const Tensor& uniqueInverse, const Tensor& uniqueOffset, int64_t tableId)
     {
-        enqueue_out(globalIds, hashIndices, offset, unique, uniqueIds, uniqueInverse, uniqueOffset, tableId);
+        enqueue_tables({this}, globalIds, hashIndices, offset, unique, uniqueIds,
+                       uniqueInverse, uniqueOffset, tableId);
         raise_on_status(status_, "ids2indices_unique_out");
     }
 
@@ -531,15 +536,15 @@ public:
                                       const Tensor& hashIndices, const Tensor& offsets, const Tensor& unique,
                                       const Tensor& uniqueIds, const Tensor& uniqueInverse, const Tensor& uniqueOffset)
     {
-        for (size_t t = 0; t < mappers.size(); ++t) {
-            const c10::intrusive_ptr<IdsMapperT> m = mappers.get(t);
-            m->enqueue_out(globalIds, hashIndices, offsets, unique, uniqueIds, uniqueInverse, uniqueOffset,
-                           static_cast<int64_t>(t));
-        }
-        for (size_t t = 0; t < mappers.size(); ++t) {
-            const c10::intrusive_ptr<IdsMapperT> m = mappers.get(t);
-            raise_on_status(m->status_, "parallel_ids2indices_unique_out");
-        }
+        const int64_t tables = static_cast<int64_t>(mappers.size());
+        if (tables == 0) return;
+        std::vector<IdsMapperT*> ms;
+        for (int64_t t = 0; t < tables; ++t) ms.push_back(mappers.get(t).get());
+        const Tensor status_all = enqueue_tables(ms, globalIds, hashIndices, offsets, unique, uniqueIds,
+                                                 uniqueInverse, uniqueOffset, 0).cpu();
+        for (int64_t t = 0; t < tables; ++t)
+            raise_on_status_words(status_all.data_ptr<int64_t>() + t * RECSDK_STATUS_WORDS, mappers.get(t)->status_,
+                                  "parallel_ids2indices_unique_out");
     }
 
     int64_t size() { return counters_.cpu().data_ptr<int64_t>()[0]; }
@@ -551,8 +556,10 @@ private:
         if (!ws_.defined() || ws_.numel() < need) ws_ = at::empty({need}, table_.options().dtype(at::kByte));
         return ws_;
     }
-    void enqueue_out(const Tensor& globalIds, const Tensor& hashIndices, const Tensor& offset, const Tensor& unique,
-                     const Tensor& uniqueIds, const Tensor& uniqueInverse, const Tensor& uniqueOffset, int64_t tableId)
+    // tables firstTable.. of a batch, one mapper each; returns the status words of all of them, on the device
+    static Tensor enqueue_tables(const std::vector<IdsMapperT*>& mappers, const Tensor& globalIds,
+                                 const Tensor& hashIndices, const Tensor& offset, const Tensor& unique, const Tensor& uniqueIds,
+                                 const Tensor& uniqueInverse, const Tensor& uniqueOffset, int64_t firstTable)
     {
         check_i64(globalIds, "globalIds");
         check_i64(hashIndices, "hashIndices");
@@ -560,15 +567,29 @@ private:
         check_i64(uniqueIds, "uniqueIds");
         check_i64(uniqueInverse, "uniqueInverse");
         check_i64(uniqueOffset, "uniqueOffset");
-        TORCH_CHECK(offset.numel() - 1 > tableId, "offset must be equal to table size + 1");
-        const Tensor off = offset.cpu();  // segment bounds are host scalars for the launch
-        const int64_t start = off.data_ptr<int64_t>()[tableId], end = off.data_ptr<int64_t>()[tableId + 1];
-        Tensor ws = workspace(end - start);
-        check_rc(recsdk_mapper_unique_out(&m_, globalIds.data_ptr<int64_t>(), hashIndices.data_ptr<int64_t>(), start,
-                                          end - start, unique.data_ptr<int64_t>(), uniqueIds.data_ptr<int64_t>(),
-                                          uniqueInverse.data_ptr<int64_t>(), uniqueOffset.data_ptr<int64_t>(), tableId,
-                                          status_.data_ptr<int64_t>(), ws.data_ptr(), ws.numel(), cur_stream()),
+        const int64_t tables = static_cast<int64_t>(mappers.size());
+        TORCH_CHECK(offset.numel() - 1 > firstTable + tables - 1, "offset must be equal to table size + 1");
+        const Tensor off = offset.cpu();  // segment bounds are host scalars for the launches
+        const int64_t* seg = off.data_ptr<int64_t>() + firstTable;
+        std::vector<const recsdk_mapper_t*> ms(tables);
+        std::vector<int64_t*> status(tables);
+        std::vector<void*> ws(tables);
+        std::vector<size_t> ws_bytes(tables);
+        for (int64_t t = 0; t < tables; ++t) {
+            const Tensor w = mappers[t]->workspace(seg[t + 1] - seg[t]);
+            ms[t] = &mappers[t]->m_;
+            status[t] = mappers[t]->status_.template data_ptr<int64_t>();
+            ws[t] = w.data_ptr();
+            ws_bytes[t] = w.numel();
+        }
+        Tensor status_all = at::empty({(firstTable + tables) * RECSDK_STATUS_WORDS}, globalIds.options());
+        check_rc(recsdk_mapper_unique_out_multi(ms.data(), tables, firstTable, globalIds.data_ptr<int64_t>(),
+                                                hashIndices.data_ptr<int64_t>(), seg, unique.data_ptr<int64_t>(),
+                                                uniqueIds.data_ptr<int64_t>(), uniqueInverse.data_ptr<int64_t>(),
+                                                uniqueOffset.data_ptr<int64_t>(), status.data(),
+                                                status_all.data_ptr<int64_t>(), ws.data(), ws_bytes.data(), cur_stream()),
                  "ids2indices_unique_out");
+        return status_all;
     }
 
     int64_t initMaxIndex_;

@@ -122,12 +122,28 @@ class IdsMapper:
     @staticmethod
     def parallel_ids2indices_unique_out(mappers: Sequence["IdsMapper"], ids, hash_indices, offsets, unique,
                                         unique_ids, unique_inverse, unique_offset, check: bool = True) -> None:
-        """ids_mapper.cpp:227-285: one mapper per table; tables are enqueued back to back on the stream."""
-        offs = offsets.tolist() if isinstance(offsets, torch.Tensor) else list(offsets)
-        for t, m in enumerate(mappers):
-            m.ids2indices_unique_out(ids, hash_indices, offs, unique, unique_ids, unique_inverse, unique_offset, t,
-                                     check=False)
-        if check:
+        """ids_mapper.cpp:227-285: one mapper per table; the tables' phases run together, one launch per phase."""
+        _chk(ids, torch.int64, "globalIds")
+        _chk(hash_indices, torch.int64, "hashIndices")
+        _chk(unique, torch.int64, "unique")
+        _chk(unique_ids, torch.int64, "uniqueIds")
+        _chk(unique_inverse, torch.int64, "uniqueInverse")
+        _chk(unique_offset, torch.int64, "uniqueOffset")
+        offs = [int(o) for o in (offsets.tolist() if isinstance(offsets, torch.Tensor) else offsets)]
+        T = len(mappers)
+        if T == 0:
+            return
+        if not (len(offs) - 1 > T - 1):
+            raise RuntimeError("offset must be equal to table size + 1")
+        ws = [m._workspace_for(offs[t + 1] - offs[t]) for t, m in enumerate(mappers)]
+        status = torch.empty(T * _lib.STATUS_WORDS, dtype=torch.int64, device=ids.device)
+        _lib.check(mappers[0]._lib.recsdk_mapper_unique_out_multi(
+            (C.POINTER(_lib.MapperT) * T)(*[C.pointer(m._c) for m in mappers]), T, 0, _ptr(ids), _ptr(hash_indices),
+            (C.c_int64 * (T + 1))(*offs[:T + 1]), _ptr(unique), _ptr(unique_ids), _ptr(unique_inverse), _ptr(unique_offset),
+            (C.c_void_p * T)(*[m._status.data_ptr() for m in mappers]), _ptr(status),
+            (C.c_void_p * T)(*[w.data_ptr() for w in ws]), (C.c_size_t * T)(*[w.numel() for w in ws]), _stream()),
+            "parallel_ids2indices_unique_out")
+        if check and any(status[::_lib.STATUS_WORDS].tolist()):
             for m in mappers:
                 m.raise_if_error("parallel_ids2indices_unique_out")
 
