@@ -3,8 +3,8 @@
 //
 // The op is HBM-bound, but a naive "one warp per bag" mapping is latency-bound:
 // offsets -> index -> row is a chain of three dependent global loads per bag.
-// Here G lanes (G*16 bytes = one row, at most a warp) own G consecutive bags:
-//   * each lane fetches the metadata of ONE of the G bags (offsets, feature
+// Here G lanes (G*16 bytes = one row, at most a warp) own up to G consecutive bags:
+//   * each lane fetches the metadata of ONE of those bags (offsets, feature
 //     geometry) and, 32 positions at a time, ONE index of the contiguous index
 //     range those bags cover, and resolves it to a row address -- all in parallel;
 //   * the group then walks the resolved rows in order, broadcasting the row
@@ -31,6 +31,7 @@ struct FwdParams {
     int64_t w_numel;
     int64_t* status;
     int base_aligned;  // dev_weights is 16-byte aligned
+    int bags_per_group;  // consecutive bags a group takes, 1..G; 0 = G
     recsdk_sample_shards sh;  // num_shards > 0: pooled rows go to the sample owners' buffers
 };
 
@@ -52,31 +53,6 @@ __device__ __forceinline__ bool row_ok(const FwdParams& p, int64_t idx, int64_t 
     return true;
 }
 
-// Generic per-bag path (any dim / offset alignment), G lanes striding over the columns.
-template <int G>
-__device__ void forward_bag_scalar(const FwdParams& p, int lane, int64_t bag)
-{
-    const int64_t t = bag / p.B;
-    const int64_t b = bag - t * p.B;
-    const int64_t s = p.offs[bag], e = p.offs[bag + 1];
-    const int32_t d0 = p.dofs[t];
-    const int32_t D = p.dofs[t + 1] - d0;
-    const int64_t wofs = p.wofs[t];
-    float* out_row = out_row_ptr(p, t, b, d0);
-    const float mean = __fdiv_rn(1.0f, static_cast<float>(e - s));
-    for (int c = lane; c < D; c += G) {
-        float acc = 0.f;
-        for (int64_t i = s; i < e; ++i) {
-            int64_t id = p.idx[i];
-            int64_t ro = wofs + id * D;
-            float v = row_ok(p, id, ro, D) ? p.w[ro + c] : 0.f;
-            acc = __fadd_rn(acc, v);
-        }
-        if (p.mode == RECSDK_POOL_MEAN && e > s) acc = __fmul_rn(acc, mean);
-        out_row[c] = acc;
-    }
-}
-
 template <int G>
 __device__ __forceinline__ unsigned group_mask()
 {
@@ -84,128 +60,148 @@ __device__ __forceinline__ unsigned group_mask()
     return ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
 }
 
-// Independent 128-bit row loads in flight per lane (divided by K).  4, not 8: at 8 the kernel needs 96 registers
+// Independent row loads in flight per lane (divided by K).  4, not 8: at 8 the kernel needs 96 registers
 // and two blocks per SM, at 4 it needs 64 and runs four -- the pooled gather of the benchmark went from 0.30 to
 // 0.22 ms.
 constexpr int kFwdUnroll = 4;
 
+// What lane j of a group knows about the j-th of the group's bags.
+struct BagLane {
+    int64_t start, wofs, optr;
+    int32_t D;
+};
+
+// The group walks the ids of its nb bags [p0, end_all), K vectors of V::W floats per lane and column pass, and
+// writes one pooled row per bag.
+template <typename V, int G, int K, int kUnroll>
+__device__ __forceinline__ void pooled_walk(const FwdParams& p, const BagLane& bl, int gl, unsigned gmask, int nb, int64_t p0,
+                                            int64_t end_all, int max_nvec)
+{
+    using T = typename V::T;
+    // flush bag j: write `acc` (scaled for MEAN) or zeros
+    auto flush = [&](int j, const T (&acc)[K], bool has_rows, int cb) {
+        float* optr = reinterpret_cast<float*>(__shfl_sync(gmask, bl.optr, j, G));
+        const int nvec = __shfl_sync(gmask, bl.D, j, G) / V::W;
+        float mean = 1.0f;
+        if (p.mode == RECSDK_POOL_MEAN) {
+            const int64_t sj = __shfl_sync(gmask, bl.start, j, G);
+            const int64_t nx = __shfl_sync(gmask, bl.start, (j + 1) & (G - 1), G);
+            mean = __fdiv_rn(1.0f, static_cast<float>(((j + 1 < nb) ? nx : end_all) - sj));
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int c = cb + gl + k * G;
+            if (c < nvec) {
+                T r = has_rows ? acc[k] : V::zero();
+                if (has_rows && p.mode == RECSDK_POOL_MEAN) r = mul4s(r, mean);
+                V::st_stream(optr + V::W * c, r);
+            }
+        }
+    };
+
+    for (int cb = 0; cb < max_nvec; cb += G * K) {
+        int cur = 0;           // bag (0..nb) whose rows are being accumulated
+        bool cur_has = false;  // accumulator holds at least one row
+        T acc[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] = V::zero();
+
+        for (int64_t base = p0; base < end_all; base += G) {
+            const int64_t pos = base + gl;
+            const bool have = pos < end_all;
+            const int64_t id = have ? p.idx[pos] : 0;
+            // bag of `pos`: the largest j with start_j <= pos (empty bags share a start; the last owns it)
+            int j_l = 0;
+#pragma unroll
+            for (int step = G >> 1; step >= 1; step >>= 1) {
+                const int cand = j_l + step;
+                const int64_t sc = __shfl_sync(gmask, bl.start, cand & (G - 1), G);
+                if (cand < G && sc <= pos) j_l = cand;
+            }
+            const int64_t wofs_j = __shfl_sync(gmask, bl.wofs, j_l, G);
+            const int32_t D_j = __shfl_sync(gmask, bl.D, j_l, G);
+            int64_t ro_l = wofs_j + id * D_j;
+            if (have && !row_ok(p, id, ro_l, D_j)) ro_l = -1;
+            const int cnt = static_cast<int>((end_all - base) < G ? (end_all - base) : G);
+
+            for (int jj0 = 0; jj0 < cnt; jj0 += kUnroll) {
+                T v[kUnroll][K];
+                int bj[kUnroll];
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    const int jj = jj0 + u;
+                    const int src = jj < cnt ? jj : 0;
+                    const int64_t ro = __shfl_sync(gmask, ro_l, src, G);
+                    bj[u] = __shfl_sync(gmask, j_l, src, G);
+                    const int nvec = __shfl_sync(gmask, bl.D, bj[u], G) / V::W;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const int c = cb + gl + k * G;
+                        v[u][k] = (jj < cnt && ro >= 0 && c < nvec) ? V::ld(p.w + ro + V::W * c) : V::zero();
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    if (jj0 + u < cnt) {
+                        while (cur < bj[u]) {  // group-uniform: finished (or empty) bags
+                            flush(cur, acc, cur_has, cb);
+#pragma unroll
+                            for (int k = 0; k < K; ++k) acc[k] = V::zero();
+                            cur_has = false;
+                            ++cur;
+                        }
+#pragma unroll
+                        for (int k = 0; k < K; ++k) acc[k] = add4(acc[k], v[u][k]);
+                        cur_has = true;
+                    }
+                }
+            }
+        }
+        while (cur < nb) {
+            flush(cur, acc, cur_has, cb);
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc[k] = V::zero();
+            cur_has = false;
+            ++cur;
+        }
+    }
+}
+
+// Latency decides wherever the bags do not fill the chip, so a group takes as many bags (p.bags_per_group <= G) as
+// leave every SM several waves of groups; see bags_per_group().
 template <int G, int K>
-__global__ void __launch_bounds__(256) tbe_forward_pooled_kernel(FwdParams p)
+__global__ void __launch_bounds__(256, K == 4 ? 3 : 4) tbe_forward_pooled_kernel(FwdParams p)
 {
     const int gl = threadIdx.x % G;
     const unsigned gmask = group_mask<G>();
     const int64_t num_bags = p.T * p.B;
     const int64_t groups_total = static_cast<int64_t>(gridDim.x) * blockDim.x / G;
     const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / G;
-    const int max_nvec = p.max_D >> 2;
+    const int per = p.bags_per_group > 0 ? p.bags_per_group : G;
 
-    for (int64_t bag0 = gid * G; bag0 < num_bags; bag0 += groups_total * G) {
-        const int nb = static_cast<int>((num_bags - bag0) < G ? (num_bags - bag0) : G);
+    for (int64_t bag0 = gid * per; bag0 < num_bags; bag0 += groups_total * per) {
+        const int nb = static_cast<int>((num_bags - bag0) < per ? (num_bags - bag0) : per);
         const bool valid = gl < nb;
         const int64_t my_bag = bag0 + gl;
-        const int64_t start_l = valid ? p.offs[my_bag] : INT64_MAX;
+        BagLane bl;
+        bl.start = valid ? p.offs[my_bag] : INT64_MAX;
         const int64_t end_all = p.offs[bag0 + nb];
         const int64_t t_l = valid ? my_bag / p.B : 0;
         const int64_t b_l = my_bag - t_l * p.B;
         const int32_t d0_l = p.dofs[t_l];
-        const int32_t D_l = p.dofs[t_l + 1] - d0_l;
-        const int64_t wofs_l = p.wofs[t_l];
-        const int64_t optr_l = valid ? reinterpret_cast<int64_t>(out_row_ptr(p, t_l, b_l, d0_l)) : 0;
-        const bool ok_l = !valid || ((((wofs_l | D_l) & 3) == 0) && ((optr_l & 15) == 0));
+        bl.D = p.dofs[t_l + 1] - d0_l;
+        bl.wofs = p.wofs[t_l];
+        bl.optr = valid ? reinterpret_cast<int64_t>(out_row_ptr(p, t_l, b_l, d0_l)) : 0;
+        const bool ok_l = !valid || ((((bl.wofs | bl.D) & 3) == 0) && ((bl.optr & 15) == 0));
         const bool all_ok = __all_sync(gmask, ok_l) != 0;  // executed by every lane of the group
-        if (!(p.base_aligned && all_ok)) {
-            for (int j = 0; j < nb; ++j) forward_bag_scalar<G>(p, gl, bag0 + j);
-            continue;
-        }
-        const int64_t p0 = __shfl_sync(gmask, start_l, 0, G);
-
-        // flush bag j: write `acc` (scaled for MEAN) or zeros
-        auto flush = [&](int j, const float4 (&acc)[K], bool has_rows, int cb) {
-            float* optr = reinterpret_cast<float*>(__shfl_sync(gmask, optr_l, j, G));
-            const int nvec = __shfl_sync(gmask, D_l, j, G) >> 2;
-            const int64_t sj = __shfl_sync(gmask, start_l, j, G);
-            const int64_t nx = __shfl_sync(gmask, start_l, (j + 1) & (G - 1), G);
-            const int64_t ej = (j + 1 < nb) ? nx : end_all;
-            const float mean = __fdiv_rn(1.0f, static_cast<float>(ej - sj));
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int c = cb + gl + k * G;
-                if (c < nvec) {
-                    float4 r = has_rows ? acc[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (has_rows && p.mode == RECSDK_POOL_MEAN) r = mul4s(r, mean);
-                    st_f4_stream(optr + 4 * c, r);
-                }
-            }
-        };
-
-        for (int cb = 0; cb < max_nvec; cb += G * K) {
-            int cur = 0;           // bag (0..nb) whose rows are being accumulated
-            bool cur_has = false;  // accumulator holds at least one row
-            float4 acc[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-
-            for (int64_t base = p0; base < end_all; base += G) {
-                const int64_t pos = base + gl;
-                const bool have = pos < end_all;
-                const int64_t id = have ? p.idx[pos] : 0;
-                // bag of `pos`: the largest j with start_j <= pos (empty bags share a start; the last owns it)
-                int j_l = 0;
-#pragma unroll
-                for (int step = G >> 1; step >= 1; step >>= 1) {
-                    const int cand = j_l + step;
-                    const int64_t sc = __shfl_sync(gmask, start_l, cand & (G - 1), G);
-                    if (cand < G && sc <= pos) j_l = cand;
-                }
-                const int64_t wofs_j = __shfl_sync(gmask, wofs_l, j_l, G);
-                const int32_t D_j = __shfl_sync(gmask, D_l, j_l, G);
-                int64_t ro_l = wofs_j + id * D_j;
-                if (have && !row_ok(p, id, ro_l, D_j)) ro_l = -1;
-                const int cnt = static_cast<int>((end_all - base) < G ? (end_all - base) : G);
-
-                constexpr int kUnroll = kFwdUnroll / K;  // independent row loads in flight per lane
-                for (int jj0 = 0; jj0 < cnt; jj0 += kUnroll) {
-                    float4 v[kUnroll][K];
-                    int bj[kUnroll];
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        const int jj = jj0 + u;
-                        const int src = jj < cnt ? jj : 0;
-                        const int64_t ro = __shfl_sync(gmask, ro_l, src, G);
-                        bj[u] = __shfl_sync(gmask, j_l, src, G);
-                        const int nvec = __shfl_sync(gmask, D_l, bj[u], G) >> 2;
-#pragma unroll
-                        for (int k = 0; k < K; ++k) {
-                            const int c = cb + gl + k * G;
-                            v[u][k] = (jj < cnt && ro >= 0 && c < nvec) ? ld_f4(p.w + ro + 4 * c)
-                                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        if (jj0 + u < cnt) {
-                            while (cur < bj[u]) {  // group-uniform: finished (or empty) bags
-                                flush(cur, acc, cur_has, cb);
-#pragma unroll
-                                for (int k = 0; k < K; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                cur_has = false;
-                                ++cur;
-                            }
-#pragma unroll
-                            for (int k = 0; k < K; ++k) acc[k] = add4(acc[k], v[u][k]);
-                            cur_has = true;
-                        }
-                    }
-                }
-            }
-            while (cur < nb) {
-                flush(cur, acc, cur_has, cb);
-#pragma unroll
-                for (int k = 0; k < K; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                cur_has = false;
-                ++cur;
-            }
-        }
+        const int64_t p0 = __shfl_sync(gmask, bl.start, 0, G);
+        // table and output rows that lie on 16 bytes move as 128-bit vectors, all others word by word, four words per lane and row
+        // (the same bytes in flight); both walks keep several rows in flight.  Eleven tables of widths 8..128 with
+        // one of 18, 3001 samples: 155 us when the second walk took one id and one word at a time, now 38.
+        if (p.base_aligned && all_ok)
+            pooled_walk<V4, G, K, kFwdUnroll / K>(p, bl, gl, gmask, nb, p0, end_all, p.max_D >> 2);
+        else
+            pooled_walk<V1, G, 4, kFwdUnroll>(p, bl, gl, gmask, nb, p0, end_all, p.max_D);
     }
 }
 
@@ -244,14 +240,27 @@ __global__ void __launch_bounds__(256) tbe_forward_nobag_kernel(FwdParams p)
 }
 
 #ifndef RECSDK_EMULATE  // host side: not part of host-side SIMT emulation builds (tests/emu)
+// Bags per group: a power of two, G (coalesced metadata, one lane per bag) only while that still leaves two waves of
+// resident groups (1024 threads per SM at 64 registers).  With G always: 962 bags of up to 10 rows of 128 floats were
+// 30 warps on 148 SMs and took 29.5 us, now 4.1; 98304 bags of up to 30 rows of 256 floats were 0.65 waves, 231 us,
+// now 177.  (Four waves instead of two: 174 against 177 us there, 0.4 % slower on 425984 bags of up to 100 rows of 64 floats.)
+static int bags_per_group(int64_t num_bags, int G)
+{
+    const int64_t two_waves = static_cast<int64_t>(num_sms()) * (1024 / G) * 2;
+    int per = 1;
+    while (per < G && static_cast<int64_t>(per) * 2 * two_waves <= num_bags) per <<= 1;
+    return per;
+}
+
 template <int G, int K>
-static void launch_pooled(const FwdParams& p, bool leave_room, cudaStream_t st)
+static void launch_pooled(FwdParams p, bool leave_room, cudaStream_t st)
 {
     const int groups_per_block = 256 / G;
+    p.bags_per_group = bags_per_group(p.T * p.B, G);
     // several waves of short-lived blocks rather than one resident wave: when the backward's index kernels run
     // beside this one on another stream, their blocks get SM slots as these retire (measured: 16 per SM 0.833 ms
     // per benchmark step, 8: 0.838, 2: 0.873; alone the grid size makes no difference)
-    int grid = grid_for(ceil_div(p.T * p.B, G), groups_per_block, 16);
+    int grid = grid_for(ceil_div(p.T * p.B, p.bags_per_group), groups_per_block, 16);
     size_t smem = 0;
     if (leave_room) {
         // unused dynamic shared memory as an occupancy limit: 60 KB per block -> three blocks per SM
@@ -290,7 +299,7 @@ extern "C" int recsdk_tbe_forward(const recsdk_tbe_forward_args* a, void* stream
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     FwdParams p{a->dev_weights, a->weights_offsets, a->D_offsets, a->indices, a->offsets, a->out, a->T, a->B, a->N,
                 a->total_D, a->max_D, a->pooling_mode, a->weights_numel, a->dev_status,
-                aligned16(a->dev_weights) ? 1 : 0, sh};
+                aligned16(a->dev_weights) ? 1 : 0, 0, sh};
     const int vec_per_row = (a->max_D + 3) / 4;
     const int G = group_lanes_for(vec_per_row);
     const bool leave_room = (a->flags & RECSDK_FWD_LEAVE_ROOM) != 0;
