@@ -766,4 +766,160 @@ static inline int radix_sort_pairs_big(KeyT* keys_a, uint32_t* vals_a, KeyT* key
     return cur;
 }
 
+// ----------------------------------------------------------------------------
+// Stable sort of the n <= THREADS * ITEMS pairs in shared memory by the key bits [0, key_bits), 8 at a time; digits in
+// which all keys agree are skipped.  A pass is a rank inside the warps (32 consecutive positions a round), a prefix
+// over the warps per digit, and a move in shared memory.  wcnt: [THREADS / 32][256], dbase: 256 ints, sm: 33 ints.
+// Called by all threads; the pairs are complete on entry (after a barrier) and on return.
+// ----------------------------------------------------------------------------
+template <typename KeyT, int THREADS, int ITEMS>
+__device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uint16_t* wcnt, int* dbase, int* sm, int n,
+                                                 int key_bits)
+{
+    constexpr int RADIX = 256, WARPS = THREADS / 32;
+    static_assert(THREADS >= RADIX, "one thread per digit");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rounds = (n + THREADS - 1) / THREADS;
+    const int first = warp * rounds * 32 + lane;
+    uint16_t* mine = wcnt + warp * RADIX;
+    for (int shift = 0; shift < key_bits; shift += 8) {
+        KeyT key[ITEMS];
+        uint32_t val[ITEMS];
+        int rank[ITEMS];
+        const unsigned digit0 = static_cast<unsigned>(skey[0] >> shift) & (RADIX - 1);
+        int differs = 0;
+        for (int w = threadIdx.x; w < WARPS * RADIX / 2; w += THREADS) reinterpret_cast<uint32_t*>(wcnt)[w] = 0;
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (r < rounds && first + r * 32 < n) {
+                key[r] = skey[first + r * 32];
+                val[r] = sval[first + r * 32];
+                differs |= (static_cast<unsigned>(key[r] >> shift) & (RADIX - 1)) != digit0;
+            }
+        if (!__syncthreads_or(differs)) continue;
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (r < rounds) {
+                const bool valid = first + r * 32 < n;
+                const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & (RADIX - 1) : RADIX + lane;
+                const unsigned peers = __match_any_sync(kFullMask, tag);
+                const unsigned before = __popc(peers & lanemask_lt());
+                const uint32_t prev = valid ? mine[tag] : 0;
+                __syncwarp();
+                if (valid && before == 0) mine[tag] = static_cast<uint16_t>(prev + __popc(peers));
+                __syncwarp();
+                rank[r] = static_cast<int>(prev + before);
+            }
+        __syncthreads();
+        int count = 0;
+        if (threadIdx.x < RADIX) {
+#pragma unroll 8
+            for (int w = 0; w < WARPS; ++w) {
+                const int c = wcnt[w * RADIX + threadIdx.x];
+                wcnt[w * RADIX + threadIdx.x] = static_cast<uint16_t>(count);
+                count += c;
+            }
+        }
+        int all;
+        const int base = block_inclusive_scan(count, sm, &all) - count;
+        if (threadIdx.x < RADIX) dbase[threadIdx.x] = base;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (r < rounds && first + r * 32 < n) {
+                const unsigned d = static_cast<unsigned>(key[r] >> shift) & (RADIX - 1);
+                const int pos = dbase[d] + mine[d] + rank[r];
+                skey[pos] = key[r];
+                sval[pos] = val[r];
+            }
+        __syncthreads();
+    }
+}
+
+// ----------------------------------------------------------------------------
+// Merge sort of (key, position) pairs for wide keys in mid-size batches: sorted tiles of kMergeTile, then rounds that
+// merge four runs each.  In a round every pair finds its place by itself: its index in its own run plus the number of
+// pairs of the three other runs that come before it, three independent binary searches.  Bound by launches and load
+// latency at these sizes, so what counts is the number of kernels: 1 + log4(tiles) against three per 8 to 10 bits of
+// the radix sort (131072 keys of 62 bits: 4 against 22 launches).
+// ----------------------------------------------------------------------------
+constexpr int kMergeThreads = 1024;
+constexpr int kMergeItems = 2;
+constexpr int kMergeTile = kMergeThreads * kMergeItems;
+constexpr int64_t kMergeMaxN = int64_t(1) << 20;
+
+// keys and positions of one tile of ids, sorted
+template <typename KeyT>
+__global__ void __launch_bounds__(kMergeThreads) merge_tile_kernel(const int64_t* __restrict__ ids, int64_t n, int key_bits,
+                                                                   KeyT* __restrict__ keys, uint32_t* __restrict__ vals)
+{
+    __shared__ KeyT skey[kMergeTile];
+    __shared__ uint32_t sval[kMergeTile];
+    __shared__ uint16_t wcnt[kMergeThreads / 32 * 256];
+    __shared__ int dbase[256];
+    __shared__ int sm[33];
+    const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * kMergeTile;
+    const int count = n - tile0 < kMergeTile ? static_cast<int>(n - tile0) : kMergeTile;
+    for (int i = threadIdx.x; i < count; i += kMergeThreads) {
+        skey[i] = static_cast<KeyT>(ids[tile0 + i]);
+        sval[i] = static_cast<uint32_t>(tile0 + i);
+    }
+    __syncthreads();
+    block_sort_pairs<KeyT, kMergeThreads, kMergeItems>(skey, sval, wcnt, dbase, sm, count, key_bits);
+    for (int i = threadIdx.x; i < count; i += kMergeThreads) {
+        keys[tile0 + i] = skey[i];
+        vals[tile0 + i] = sval[i];
+    }
+}
+
+// runs of `run` pairs (the last may be shorter) -> runs of 4 * run
+template <typename KeyT>
+__global__ void __launch_bounds__(256) merge_round_kernel(const KeyT* __restrict__ keys, const uint32_t* __restrict__ vals,
+                                                          int64_t n, int64_t run, KeyT* __restrict__ keys_out,
+                                                          uint32_t* __restrict__ vals_out)
+{
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const KeyT key = keys[i];
+    const uint32_t val = vals[i];
+    const int64_t group0 = i / (4 * run) * (4 * run);
+    const int own = static_cast<int>((i - group0) / run);
+    int64_t lo[4], hi[4];  // in run q: number of pairs before this one lies in [lo, hi]
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int64_t start = group0 + q * run;
+        const int64_t len = start >= n ? 0 : (n - start < run ? n - start : run);
+        lo[q] = q == own ? i - start : 0;
+        hi[q] = q == own ? i - start : len;
+    }
+    for (int64_t left = run; left > 0; left >>= 1) {  // halves every interval: run + 1 outcomes take log2(run) + 1 steps
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (lo[q] < hi[q]) {
+                const int64_t mid = (lo[q] + hi[q]) >> 1;
+                const KeyT other = keys[group0 + q * run + mid];
+                // equal keys of earlier runs come first
+                if (q < own ? other <= key : other < key) lo[q] = mid + 1; else hi[q] = mid;
+            }
+        }
+    }
+    const int64_t pos = group0 + lo[0] + lo[1] + lo[2] + lo[3];
+    keys_out[pos] = key;
+    vals_out[pos] = val;
+}
+
+// ids -> pairs sorted by the key bits [0, key_bits); result in the a-buffers (0) or the b-buffers (1).  n <= kMergeMaxN.
+template <typename KeyT>
+static inline int merge_sort_ids(const int64_t* ids, int64_t n, int key_bits, KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b,
+                                 uint32_t* vals_b, cudaStream_t st)
+{
+    merge_tile_kernel<KeyT><<<static_cast<unsigned>(ceil_div(n, kMergeTile)), kMergeThreads, 0, st>>>(ids, n, key_bits, keys_a,
+                                                                                                    vals_a);
+    int cur = 0;
+    for (int64_t run = kMergeTile; run < n; run *= 4, cur ^= 1)
+        merge_round_kernel<KeyT><<<static_cast<unsigned>(ceil_div(n, 256)), 256, 0, st>>>(
+            cur ? keys_b : keys_a, cur ? vals_b : vals_a, n, run, cur ? keys_a : keys_b, cur ? vals_a : vals_b);
+    return cur;
+}
+
 }  // namespace recsdk

@@ -618,17 +618,15 @@ __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* 
 // One block does what expand, the sort passes, the run scan and the records do for a batch that fits its shared memory
 // (at most kSmallN positions in at most kSmallN bags).  Such a batch is bound by launches and by the latency of each
 // kernel's first loads, not by work: 4096 ids of 20-bit keys took eleven launches, 37 us of kernels and the gaps between them, against 25 us
-// in this one launch (a training step of them 116 -> 93..102 us).  A radix pass is a rank inside the warps (32 consecutive positions a round), a prefix
-// over the warps per digit, and a move in shared memory: stable, like the passes of the large sorts.
+// in this one launch (a training step of them 116 -> 93..102 us).  
 constexpr int kSmallN = 8192;
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallItems = kSmallN / kSmallThreads;
-constexpr int kSmallBits = 8;
 template <typename KeyT>
 constexpr size_t plan_small_smem()
 {
     return kSmallN * (sizeof(KeyT) + sizeof(uint32_t)) + (kSmallN + 4) * sizeof(int) +
-           (kSmallThreads / 32) * (size_t(1) << kSmallBits) * sizeof(uint16_t);
+           (kSmallThreads / 32) * 256 * sizeof(uint16_t);
 }
 
 template <typename KeyT>
@@ -636,13 +634,13 @@ __global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, 
                                                                    int* __restrict__ run_start, int64_t* counters,
                                                                    RunMeta* __restrict__ meta, int2* __restrict__ desc)
 {
-    constexpr int RADIX = 1 << kSmallBits, WARPS = kSmallThreads / 32;
+    constexpr int WARPS = kSmallThreads / 32;
     extern __shared__ __align__(16) unsigned char small_smem[];
     __shared__ int sm[33];
     KeyT* skey = reinterpret_cast<KeyT*>(small_smem);
     uint32_t* sval = reinterpret_cast<uint32_t*>(skey + kSmallN);
     int* srun = reinterpret_cast<int*>(sval + kSmallN);
-    uint16_t* wcnt = reinterpret_cast<uint16_t*>(srun + kSmallN + 4);  // [WARPS][RADIX]
+    uint16_t* wcnt = reinterpret_cast<uint16_t*>(srun + kSmallN + 4);  // [WARPS][256]
     const int n = static_cast<int>(p.N);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < n; i += kSmallThreads) {
@@ -668,58 +666,8 @@ __global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, 
             });
     }
     __syncthreads();
+    block_sort_pairs<KeyT, kSmallThreads, kSmallItems>(skey, sval, wcnt, srun, sm, n, key_bits);
     const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
-    const int first = warp * rounds * 32 + lane;
-    uint16_t* mine = wcnt + warp * RADIX;
-    for (int shift = 0; shift < key_bits; shift += kSmallBits) {
-        KeyT key[kSmallItems];
-        uint32_t val[kSmallItems];
-        int rank[kSmallItems];
-        for (int w = threadIdx.x; w < WARPS * RADIX / 2; w += kSmallThreads) reinterpret_cast<uint32_t*>(wcnt)[w] = 0;
-#pragma unroll
-        for (int r = 0; r < kSmallItems; ++r)
-            if (r < rounds && first + r * 32 < n) {
-                key[r] = skey[first + r * 32];
-                val[r] = sval[first + r * 32];
-            }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kSmallItems; ++r)
-            if (r < rounds) {
-                const bool valid = first + r * 32 < n;
-                const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & (RADIX - 1) : RADIX + lane;
-                const unsigned peers = __match_any_sync(kFullMask, tag);
-                const unsigned before = __popc(peers & lanemask_lt());
-                const uint32_t prev = valid ? mine[tag] : 0;
-                __syncwarp();
-                if (valid && before == 0) mine[tag] = static_cast<uint16_t>(prev + __popc(peers));
-                __syncwarp();
-                rank[r] = static_cast<int>(prev + before);
-            }
-        __syncthreads();
-        int count = 0;
-        if (threadIdx.x < RADIX) {
-#pragma unroll 8
-            for (int w = 0; w < WARPS; ++w) {
-                const int c = wcnt[w * RADIX + threadIdx.x];
-                wcnt[w * RADIX + threadIdx.x] = static_cast<uint16_t>(count);
-                count += c;
-            }
-        }
-        int all;
-        const int base = block_inclusive_scan(count, sm, &all) - count;
-        if (threadIdx.x < RADIX) srun[threadIdx.x] = base;
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kSmallItems; ++r)
-            if (r < rounds && first + r * 32 < n) {
-                const unsigned d = static_cast<unsigned>(key[r] >> shift) & (RADIX - 1);
-                const int pos = srun[d] + mine[d] + rank[r];
-                skey[pos] = key[r];
-                sval[pos] = val[r];
-            }
-        __syncthreads();
-    }
     // run starts: each thread looks at `rounds` consecutive positions
     {
         const int i0 = threadIdx.x * rounds;

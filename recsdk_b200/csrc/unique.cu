@@ -1,4 +1,4 @@
-// Sorted unique + inverse of int64 ids (radix sort of (id, position) pairs,
+// Sorted unique + inverse of int64 ids (sort of (id, position) pairs,
 // adjacent-difference head flags, scan).  Same result as a CPU sort followed by
 // an adjacent-diff pass: unique ascending, inverse[i] = rank of ids[i].
 #include "prims.cuh"
@@ -16,35 +16,30 @@ __global__ void __launch_bounds__(256) unique_load_kernel(const int64_t* __restr
     }
 }
 
+// The heads of the runs are the unique ids; flags are computed and ranks consumed inside the scan.
 template <typename KeyT>
-__global__ void __launch_bounds__(256) unique_flag_kernel(const KeyT* __restrict__ keys, int64_t n, int* __restrict__ flag)
-{
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        flag[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-}
-
+struct UniqueHeadIn {
+    const KeyT* keys;
+    __device__ __forceinline__ int operator()(int64_t i) const { return (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0; }
+};
 template <typename KeyT>
-__global__ void __launch_bounds__(256) unique_write_kernel(const KeyT* __restrict__ keys,
-                                                           const uint32_t* __restrict__ vals,
-                                                           const int* __restrict__ incl, int64_t n,
-                                                           int64_t* __restrict__ unique_out,
-                                                           int64_t* __restrict__ inverse_out,
-                                                           int64_t* __restrict__ num_unique_out)
-{
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int r = incl[i] - 1;
-        if (i == 0 || keys[i] != keys[i - 1]) unique_out[r] = static_cast<int64_t>(keys[i]);
+struct UniqueOut {
+    const KeyT* keys;
+    const uint32_t* vals;
+    int64_t *unique_out, *inverse_out, *num_unique_out;
+    __device__ __forceinline__ void operator()(int64_t i, int head, int incl, int64_t n) const
+    {
+        const int r = incl - 1;
+        if (head) unique_out[r] = static_cast<int64_t>(keys[i]);
         inverse_out[vals[i]] = r;
-        if (i == n - 1 && num_unique_out != nullptr) *num_unique_out = r + 1;
+        if (i == n - 1 && num_unique_out != nullptr) *num_unique_out = incl;
     }
-}
+};
 
 struct UniqueWorkspace {
     void *keys_a, *keys_b;
     uint32_t *vals_a, *vals_b, *sort_scratch;
-    int *flag, *scan_scratch;
+    int* scan_scratch;
     size_t bytes;
 };
 
@@ -58,11 +53,15 @@ static UniqueWorkspace carve_unique(void* base, int64_t N)
     w.vals_a = c.take<uint32_t>(n);
     w.vals_b = c.take<uint32_t>(n);
     w.sort_scratch = c.take<uint32_t>(sort_scratch_u32(N));
-    w.flag = c.take<int>(n);
     w.scan_scratch = c.take<int>(scan_scratch_ints(N));
     w.bytes = c.used();
     return w;
 }
+
+// Keys wider than this take the merge sort (up to its size limit): its rounds depend on n alone, the radix sort's passes
+// on the bits.  131072 keys: 25 launches with 152 us in them by seven radix passes of
+// 10 bits, 6 launches merged, and the cached-table step around them 1.0 -> 0.85 ms; up to 20 bits are two passes.
+constexpr int kMergeMinBits = 20;
 
 template <typename KeyT>
 static int run_unique(const int64_t* ids, int64_t n, int key_bits, int64_t* unique_out, int64_t* inverse_out,
@@ -70,14 +69,19 @@ static int run_unique(const int64_t* ids, int64_t n, int key_bits, int64_t* uniq
 {
     KeyT* ka = static_cast<KeyT*>(ws.keys_a);
     KeyT* kb = static_cast<KeyT*>(ws.keys_b);
-    const int grid = grid_for(n, 256);
-    unique_load_kernel<KeyT><<<grid, 256, 0, st>>>(ids, n, ka, ws.vals_a);
-    const int which = radix_sort_pairs<KeyT>(ka, ws.vals_a, kb, ws.vals_b, n, key_bits, ws.sort_scratch, st);
+    int which;
+    if (key_bits > kMergeMinBits && n <= kMergeMaxN) {
+        which = merge_sort_ids<KeyT>(ids, n, key_bits, ka, ws.vals_a, kb, ws.vals_b, st);
+    } else {
+        unique_load_kernel<KeyT><<<grid_for(n, 256), 256, 0, st>>>(ids, n, ka, ws.vals_a);
+        which = radix_sort_is_big<KeyT>(n, key_bits)
+                    ? radix_sort_pairs_big<KeyT>(ka, ws.vals_a, kb, ws.vals_b, n, key_bits, ws.sort_scratch, st)
+                    : radix_sort_pairs<KeyT>(ka, ws.vals_a, kb, ws.vals_b, n, key_bits, ws.sort_scratch, st);
+    }
     const KeyT* keys = which ? kb : ka;
     const uint32_t* vals = which ? ws.vals_b : ws.vals_a;
-    unique_flag_kernel<KeyT><<<grid, 256, 0, st>>>(keys, n, ws.flag);
-    device_scan<true>(ws.flag, ws.flag, n, ws.scan_scratch, nullptr, st);
-    unique_write_kernel<KeyT><<<grid, 256, 0, st>>>(keys, vals, ws.flag, n, unique_out, inverse_out, num_unique_out);
+    device_scan_fn<true>(UniqueHeadIn<KeyT>{keys}, UniqueOut<KeyT>{keys, vals, unique_out, inverse_out, num_unique_out}, n,
+                         ws.scan_scratch, nullptr, st);
     RECSDK_CUDA_CHECK_LAUNCH();
     return RECSDK_OK;
 }
