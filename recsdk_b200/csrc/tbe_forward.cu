@@ -73,7 +73,10 @@ struct BagLane {
 
 // The group walks the ids of its nb bags [p0, end_all), K vectors of V::W floats per lane and column pass, and
 // writes one pooled row per bag.
-template <typename V, int G, int K, int kUnroll>
+// LONG (bags of several ids): a block of G resolved rows is walked bag by bag, so that the inner loop needs per row no
+// more than the shuffle of its address, the load and the adds; the other form checks every row for the end of its bag,
+// which costs more instructions but keeps kUnroll rows in flight across bags of one or two ids.
+template <typename V, int G, int K, int kUnroll, bool LONG>
 __device__ __forceinline__ void pooled_walk(const FwdParams& p, const BagLane& bl, int gl, unsigned gmask, int nb, int64_t p0,
                                             int64_t end_all, int max_nvec)
 {
@@ -124,6 +127,43 @@ __device__ __forceinline__ void pooled_walk(const FwdParams& p, const BagLane& b
             if (have && !row_ok(p, id, ro_l, D_j)) ro_l = -1;
             const int cnt = static_cast<int>((end_all - base) < G ? (end_all - base) : G);
 
+            if (LONG) {
+                for (int q = 0; q < cnt;) {
+                    const int bag = __shfl_sync(gmask, j_l, q, G);
+                    while (cur < bag) {  // group-uniform: finished (or empty) bags
+                        flush(cur, acc, cur_has, cb);
+#pragma unroll
+                        for (int k = 0; k < K; ++k) acc[k] = V::zero();
+                        cur_has = false;
+                        ++cur;
+                    }
+                    cur_has = true;
+                    const int64_t next_start = __shfl_sync(gmask, bl.start, (bag + 1) & (G - 1), G);
+                    const int64_t bag_end = bag + 1 < nb ? next_start : end_all;
+                    const int seg = bag_end - base < cnt ? static_cast<int>(bag_end - base) : cnt;
+                    const int nvec = __shfl_sync(gmask, bl.D, bag, G) / V::W;
+                    for (; q < seg; q += kUnroll) {
+                        T v[kUnroll][K];
+#pragma unroll
+                        for (int u = 0; u < kUnroll; ++u) {
+                            const int64_t ro = __shfl_sync(gmask, ro_l, (q + u) & (G - 1), G);
+#pragma unroll
+                            for (int k = 0; k < K; ++k) {
+                                const int c = cb + gl + k * G;
+                                v[u][k] = (q + u < seg && ro >= 0 && c < nvec) ? V::ld(p.w + ro + V::W * c) : V::zero();
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < kUnroll; ++u)
+                            if (q + u < seg) {
+#pragma unroll
+                                for (int k = 0; k < K; ++k) acc[k] = add4(acc[k], v[u][k]);
+                            }
+                    }
+                    q = seg;
+                }
+                continue;
+            }
             for (int jj0 = 0; jj0 < cnt; jj0 += kUnroll) {
                 T v[kUnroll][K];
                 int bj[kUnroll];
@@ -169,7 +209,7 @@ __device__ __forceinline__ void pooled_walk(const FwdParams& p, const BagLane& b
 
 // Latency decides wherever the bags do not fill the chip, so a group takes as many bags (p.bags_per_group <= G) as
 // leave every SM several waves of groups; see bags_per_group().
-template <int G, int K>
+template <int G, int K, bool LONG = false>
 __global__ void __launch_bounds__(256, K == 4 ? 3 : 4) tbe_forward_pooled_kernel(FwdParams p)
 {
     const int gl = threadIdx.x % G;
@@ -199,9 +239,9 @@ __global__ void __launch_bounds__(256, K == 4 ? 3 : 4) tbe_forward_pooled_kernel
         // (the same bytes in flight); both walks keep several rows in flight.  Eleven tables of widths 8..128 with
         // one of 18, 3001 samples: 155 us when the second walk took one id and one word at a time, now 38.
         if (p.base_aligned && all_ok)
-            pooled_walk<V4, G, K, kFwdUnroll / K>(p, bl, gl, gmask, nb, p0, end_all, p.max_D >> 2);
+            pooled_walk<V4, G, K, kFwdUnroll / K, LONG>(p, bl, gl, gmask, nb, p0, end_all, p.max_D >> 2);
         else
-            pooled_walk<V1, G, 4, kFwdUnroll>(p, bl, gl, gmask, nb, p0, end_all, p.max_D);
+            pooled_walk<V1, G, 4, kFwdUnroll, LONG>(p, bl, gl, gmask, nb, p0, end_all, p.max_D);
     }
 }
 
@@ -240,17 +280,22 @@ __global__ void __launch_bounds__(256) tbe_forward_nobag_kernel(FwdParams p)
 }
 
 #ifndef RECSDK_EMULATE  // host side: not part of host-side SIMT emulation builds (tests/emu)
-// Bags per group: a power of two, G (coalesced metadata, one lane per bag) only while that still leaves two waves of
+// Bags per group: a power of two, G (coalesced metadata, one lane per bag) only while that still leaves four waves of
 // resident groups (1024 threads per SM at 64 registers).  With G always: 962 bags of up to 10 rows of 128 floats were
 // 30 warps on 148 SMs and took 29.5 us, now 4.1; 98304 bags of up to 30 rows of 256 floats were 0.65 waves, 231 us,
-// now 177.  (Four waves instead of two: 174 against 177 us there, 0.4 % slower on 425984 bags of up to 100 rows of 64 floats.)
+// now 174 (161 with the bag-by-bag walk).  (Two waves instead of four: 177 against 174 us there.)
 static int bags_per_group(int64_t num_bags, int G)
 {
-    const int64_t two_waves = static_cast<int64_t>(num_sms()) * (1024 / G) * 2;
+    const int64_t four_waves = static_cast<int64_t>(num_sms()) * (1024 / G) * 4;
     int per = 1;
-    while (per < G && static_cast<int64_t>(per) * 2 * two_waves <= num_bags) per <<= 1;
+    while (per < G && static_cast<int64_t>(per) * 2 * four_waves <= num_bags) per <<= 1;
     return per;
 }
+
+// Ids per bag, on average, from which the bag-by-bag walk takes over: 98304 bags of
+// 15.5 rows of 256 floats 174 -> 161 us, a training step of 20 M ids in bags of 50 2984 -> 2970 us.  Bags of one or two ids
+// need the other walk to have several rows in flight; eight are two of its steps.
+constexpr int64_t kLongBagIds = 8;
 
 template <int G, int K>
 static void launch_pooled(FwdParams p, bool leave_room, cudaStream_t st)
@@ -262,12 +307,14 @@ static void launch_pooled(FwdParams p, bool leave_room, cudaStream_t st)
     // per benchmark step, 8: 0.838, 2: 0.873; alone the grid size makes no difference)
     int grid = grid_for(ceil_div(p.T * p.B, p.bags_per_group), groups_per_block, 16);
     size_t smem = 0;
-    if (leave_room) {
+    auto launch = [&](auto kernel, bool* optin_done) {
         // unused dynamic shared memory as an occupancy limit: 60 KB per block -> three blocks per SM
-        static bool optin_done[kMaxDevices] = {false};
-        if (smem_optin(tbe_forward_pooled_kernel<G, K>, 60 * 1024, optin_done)) smem = 60 * 1024;
-    }
-    tbe_forward_pooled_kernel<G, K><<<grid, 256, smem, st>>>(p);
+        if (leave_room && smem_optin(kernel, 60 * 1024, optin_done)) smem = 60 * 1024;
+        kernel<<<grid, 256, smem, st>>>(p);
+    };
+    static bool optin_short[kMaxDevices] = {false}, optin_long[kMaxDevices] = {false};
+    if (p.N >= kLongBagIds * p.T * p.B) launch(tbe_forward_pooled_kernel<G, K, true>, optin_long);
+    else launch(tbe_forward_pooled_kernel<G, K, false>, optin_short);
 }
 
 template <int G>
