@@ -1,0 +1,172 @@
+"""Kernels whose way of working depends on the size of the input, at the sizes where it changes and around the edges of
+their tiles: against the oracle (or numpy's sort), bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import port
+from tests.test_gpu_tbe import _t, make_case
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+# bags per group 1 .. G, the last group short; widths that leave rows or output columns off 16 bytes
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("rows,dims,B,max_len", [
+    ([50, 30], [128, 20], 19, 9),             # one bag per group
+    ([700], [8], 70_001, 2),                  # two-lane groups, whole groups
+    ([300, 200], [128, 64], 9_601, 3),        # a few bags per group
+    ([90, 60, 40], [8, 18, 64], 4_003, 5),    # rows and columns off 16 bytes
+    ([200], [512], 401, 30),                  # several vectors per lane, long bags
+    ([400, 90], [64, 64], 12_001, 40),        # long bags, several per group
+])
+def test_forward_bags_per_group(rows, dims, B, max_len, mode):
+    from recsdk_b200 import ops
+
+    c = make_case(np.random.default_rng(B), rows, dims, B, max_len, empty_frac=0.2)
+    exp = port.tbe_forward(c["w"], c["wo"], c["do"], c["indices"], c["offsets"], c["T"], B, c["total_D"], c["max_D"], mode)
+    out = ops.tbe_forward(_t(c["w"]), _t(c["wo"]), _t(c["do"]), _t(c["indices"]), _t(c["offsets"]), c["total_D"],
+                          c["max_D"], mode)
+    np.testing.assert_array_equal(out.cpu().numpy(), exp)
+
+
+def _backward_equals_oracle(indices, rows, dim, B, bits, opt=1, mode=0):
+    """One table; `indices` over B bags of equal length."""
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(indices.size)
+    offsets = np.linspace(0, indices.size, B + 1).astype(np.int64)
+    grad = rng.standard_normal((B, dim)).astype(np.float32)
+    w = rng.uniform(-0.05, 0.05, rows * dim).astype(np.float32)
+    m1 = np.full_like(w, 0.1)
+    dw, dm1 = _t(w), _t(m1)
+    wo, do, hs = np.zeros(1, np.int64), np.array([0, dim], np.int32), np.array([0, rows], np.int64)
+    port.tbe_backward(grad, w, m1, None, wo, do, hs, indices, offsets, 1, B, dim, dim, mode, opt, 0.05, 1e-8, 0.9, 0.999, 1,
+                      reduce_chunk=64)
+    ops.tbe_backward(_t(grad), dw, dm1, None, _t(wo), _t(do), _t(hs), _t(indices), _t(offsets), dim, dim, mode, opt, 0.05,
+                     1e-8, 0.9, 0.999, 1, total_hash_size_bits=bits, reduce_chunk=64)
+    np.testing.assert_array_equal(dw.cpu().numpy(), w)
+    np.testing.assert_array_equal(dm1.cpu().numpy(), m1)
+
+
+# the one-block plan (up to 8192 positions), the sort of mid-size and the sort of large batches; 32- and 64-bit keys
+@pytest.mark.parametrize("bits", [20, 27, 40])
+@pytest.mark.parametrize("n", [1, 1023, 1025, 8191, 8192, 8193, (1 << 20) - 1, (1 << 20) + 4097])
+def test_backward_plan_sizes(n, bits):
+    rng = np.random.default_rng(n)
+    _backward_equals_oracle(rng.integers(0, 60_000, n), 60_000, 4, min(n, 5_000), bits)
+
+
+# runs around the direct / chunked border, a chunk, the border above which a run's chunk sums get their own kernel
+@pytest.mark.parametrize("dim", [4, 8, 16, 32, 36, 64, 128, 18])
+def test_backward_run_lengths(dim):
+    lengths = [1, 2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 128, 129, 4095, 4096, 4097, 4161, 14_000, 16 * 64, 17 * 64 + 1]
+    ids = np.repeat(np.arange(len(lengths)), lengths)
+    rng = np.random.default_rng(dim)
+    rng.shuffle(ids)
+    assert ids.size > 32768  # the totals kernel runs
+    _backward_equals_oracle(ids, len(lengths), dim, 3_001, 8)
+    small = ids[ids < 12]
+    _backward_equals_oracle(small, len(lengths), dim, 301, 8, mode=1)
+
+
+@pytest.mark.parametrize("world", [1, 3, 64])
+@pytest.mark.parametrize("features,batch,max_len,vocab", [(1, 1, 1, 5), (3, 129, 9, 40), (5, 4_097, 6, 100_000)])
+def test_bucketize_dedup(features, batch, max_len, vocab, world):
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(world * batch)
+    lengths = rng.integers(0, max_len + 1, features * batch)
+    lengths[0] = 1
+    ids = rng.integers(0, vocab, int(lengths.sum())) * 0x1E3779B97F4A7C15 & ((1 << 63) - 1)
+    for count in (False, True):
+        el, ei, ep, ec = port.bucketize(lengths, ids, features, world, True, True, count)
+        nl, ni, perm, cnt, k = ops.bucketize(_t(lengths), _t(ids), features, world, True, count)
+        k = int(k.item())
+        assert k == ei.size
+        np.testing.assert_array_equal(nl.cpu().numpy(), el)
+        np.testing.assert_array_equal(ni.cpu().numpy()[:k], ei)
+        np.testing.assert_array_equal(perm.cpu().numpy(), ep)
+        if count:
+            np.testing.assert_array_equal(cnt.cpu().numpy()[:k], ec)
+
+
+# tiles of 2048, rounds of four runs, the size limit of the merge sort; the widths on either side of its rule
+@pytest.mark.parametrize("bits", [20, 21, 33, 64])
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 8193, 40_000, (1 << 20) + 1])
+def test_unique_sizes(n, bits):
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(n + bits)
+    top = (1 << min(bits, 63)) - 1
+    ids = np.where(rng.random(n) < 0.5, rng.integers(0, top, n, endpoint=True), rng.integers(0, 50, n))
+    ids[-1] = top
+    exp, inv = np.unique(ids, return_inverse=True)
+    uq, got, cnt = ops.unique_sorted(_t(ids), bits)
+    assert int(cnt.item()) == exp.size
+    np.testing.assert_array_equal(uq.cpu().numpy()[:exp.size], exp)
+    np.testing.assert_array_equal(got.cpu().numpy(), inv)
+
+
+# more tables than a group holds, empty segments, one mapper for two tables: as table after table
+@pytest.mark.parametrize("per_table", [[5], [0, 0], [0, 3000, 0, 1, 2049], [700] * 19 + [0, 4097]])
+@pytest.mark.parametrize("shared", [False, True])
+def test_mappers_together_equal_one_by_one(per_table, shared):
+    from recsdk_b200 import IdsMapper
+
+    T, n = len(per_table), sum(per_table)
+    rng = np.random.default_rng(n + T)
+    offs = np.concatenate([[0], np.cumsum(per_table)]).astype(np.int64)
+
+    def mappers():
+        ms = [IdsMapper(8192) for _ in range(T)]
+        if shared and T > 1:
+            ms[-1] = ms[0]
+        return ms
+
+    together, single = mappers(), mappers()
+    for _ in range(2):
+        ids = _t(rng.integers(0, 3000, n))
+        outs = []
+        for way in (0, 1):
+            hi, uq, uid, inv = (torch.zeros(max(n, 1), dtype=torch.int64, device=DEV) for _ in range(4))
+            uo = torch.zeros(T + 1, dtype=torch.int64, device=DEV)
+            if way == 0:
+                IdsMapper.parallel_ids2indices_unique_out(together, ids, hi, offs, uq, uid, inv, uo)
+            else:
+                for t in range(T):
+                    single[t].ids2indices_unique_out(ids, hi, torch.from_numpy(offs), uq, uid, inv, uo, t)
+            outs.append([x.cpu().numpy() for x in (hi, uq, uid, inv, uo)])
+        for a, b in zip(*outs):
+            np.testing.assert_array_equal(a, b)
+    assert [m.size() for m in together] == [m.size() for m in single]
+
+
+def test_mappers_together_report_the_table_that_failed():
+    from recsdk_b200 import IdsMapper
+
+    ms = [IdsMapper(64) for _ in range(3)]
+    ids = _t(np.array([1, 2, 3, -5, 4, 5], np.int64))
+    hi, uq, uid, inv = (torch.zeros(6, dtype=torch.int64, device=DEV) for _ in range(4))
+    with pytest.raises(RuntimeError, match="-5"):
+        IdsMapper.parallel_ids2indices_unique_out(ms, ids, hi, [0, 2, 4, 6], uq, uid, inv,
+                                                  torch.zeros(4, dtype=torch.int64, device=DEV))
+
+
+@pytest.mark.parametrize("D", [1, 6, 64, 132])
+@pytest.mark.parametrize("B,L", [(1, 1), (37, 7), (1_500, 33)])
+def test_jagged_dense_row_groups(B, L, D):
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(B + D)
+    lengths = rng.integers(0, L + 3, B)
+    lengths[0] = max(1, lengths[0])
+    offs = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    values = rng.standard_normal((int(offs[-1]), D)).astype(np.float32)
+    dense = ops.jagged_to_padded_dense(_t(values), [_t(offs)], L, 0.5)
+    exp = port.jagged_to_padded_dense(values, offs, L, 0.5)
+    np.testing.assert_array_equal(dense.cpu().numpy(), exp)
+    back, _ = ops.dense_to_jagged(dense, [_t(offs)], int(offs[-1]))
+    np.testing.assert_array_equal(back.cpu().numpy()[:int(offs[-1])], port.dense_to_jagged(exp, offs))
