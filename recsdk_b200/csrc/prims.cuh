@@ -42,6 +42,34 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int* smem, int* total
     return inc;
 }
 
+// Number of passes and bits per pass for keys of `key_bits` significant bits.
+static inline void radix_plan(int key_bits, int* passes, int* bits)
+{
+    const int p8 = (key_bits + 7) / 8, p9 = (key_bits + 8) / 9, p10 = (key_bits + 9) / 10;
+    *bits = 8;
+    *passes = p8;
+    if (p9 < *passes) {
+        *bits = 9;
+        *passes = p9;
+    }
+    if (p10 < *passes) {
+        *bits = 10;
+        *passes = p10;
+    }
+}
+// The key bits [0, this) are what the sorts of this file order keys of KeyT by: whole digits of radix_plan, cut at the
+// width of the key.  Keys may have bits above those (an id wider than the caller's key_bits): every sort leaves a
+// permutation then, too, and the same one.
+template <typename KeyT>
+static inline int radix_sorted_bits(int key_bits)
+{
+    int passes, bits;
+    radix_plan(key_bits, &passes, &bits);
+    const int width = 8 * static_cast<int>(sizeof(KeyT));
+    return passes * bits < width ? passes * bits : width;
+}
+
+#ifndef RECSDK_EMULATE
 // ----------------------------------------------------------------------------
 // Device-wide int32 scan: reduce per tile -> scan of tile sums (one block) ->
 // apply.  Tile = 256 threads x 8 items.
@@ -424,22 +452,6 @@ static inline void radix_sort_pass_fused(const KeyT* kin, const uint32_t* vin, K
                                                                                           hist, totals, tiles, next, n_dev);
 }
 
-// Number of passes and bits per pass for keys of `key_bits` significant bits.
-static inline void radix_plan(int key_bits, int* passes, int* bits)
-{
-    const int p8 = (key_bits + 7) / 8, p9 = (key_bits + 8) / 9, p10 = (key_bits + 9) / 10;
-    *bits = 8;
-    *passes = p8;
-    if (p9 < *passes) {
-        *bits = 9;
-        *passes = p9;
-    }
-    if (p10 < *passes) {
-        *bits = 10;
-        *passes = p10;
-    }
-}
-
 // Sorts n pairs by the key bits [0, key_bits).  Data ping-pongs between
 // (keys_a, vals_a) and (keys_b, vals_b); returns 0 when the result is in the
 // a-buffers, 1 when it is in the b-buffers.  n < 2^31.
@@ -766,15 +778,17 @@ static inline int radix_sort_pairs_big(KeyT* keys_a, uint32_t* vals_a, KeyT* key
     return cur;
 }
 
+#endif  // RECSDK_EMULATE
+
 // ----------------------------------------------------------------------------
-// Stable sort of the n <= THREADS * ITEMS pairs in shared memory by the key bits [0, key_bits), 8 at a time; digits in
+// Stable sort of the n <= THREADS * ITEMS pairs in shared memory by the key bits [0, sort_bits), 8 at a time; digits in
 // which all keys agree are skipped.  A pass is a rank inside the warps (32 consecutive positions a round), a prefix
 // over the warps per digit, and a move in shared memory.  wcnt: [THREADS / 32][256], dbase: 256 ints, sm: 33 ints.
 // Called by all threads; the pairs are complete on entry (after a barrier) and on return.
 // ----------------------------------------------------------------------------
 template <typename KeyT, int THREADS, int ITEMS>
 __device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uint16_t* wcnt, int* dbase, int* sm, int n,
-                                                 int key_bits)
+                                                 int sort_bits)
 {
     constexpr int RADIX = 256, WARPS = THREADS / 32;
     static_assert(THREADS >= RADIX, "one thread per digit");
@@ -782,11 +796,12 @@ __device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uin
     const int rounds = (n + THREADS - 1) / THREADS;
     const int first = warp * rounds * 32 + lane;
     uint16_t* mine = wcnt + warp * RADIX;
-    for (int shift = 0; shift < key_bits; shift += 8) {
+    for (int shift = 0; shift < sort_bits; shift += 8) {
+        const unsigned digit_mask = sort_bits - shift < 8 ? (1u << (sort_bits - shift)) - 1u : RADIX - 1;
         KeyT key[ITEMS];
         uint32_t val[ITEMS];
         int rank[ITEMS];
-        const unsigned digit0 = static_cast<unsigned>(skey[0] >> shift) & (RADIX - 1);
+        const unsigned digit0 = static_cast<unsigned>(skey[0] >> shift) & digit_mask;
         int differs = 0;
         for (int w = threadIdx.x; w < WARPS * RADIX / 2; w += THREADS) reinterpret_cast<uint32_t*>(wcnt)[w] = 0;
 #pragma unroll
@@ -794,14 +809,14 @@ __device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uin
             if (r < rounds && first + r * 32 < n) {
                 key[r] = skey[first + r * 32];
                 val[r] = sval[first + r * 32];
-                differs |= (static_cast<unsigned>(key[r] >> shift) & (RADIX - 1)) != digit0;
+                differs |= (static_cast<unsigned>(key[r] >> shift) & digit_mask) != digit0;
             }
         if (!__syncthreads_or(differs)) continue;
 #pragma unroll
         for (int r = 0; r < ITEMS; ++r)
             if (r < rounds) {
                 const bool valid = first + r * 32 < n;
-                const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & (RADIX - 1) : RADIX + lane;
+                const unsigned tag = valid ? static_cast<unsigned>(key[r] >> shift) & digit_mask : RADIX + lane;
                 const unsigned peers = __match_any_sync(kFullMask, tag);
                 const unsigned before = __popc(peers & lanemask_lt());
                 const uint32_t prev = valid ? mine[tag] : 0;
@@ -827,7 +842,7 @@ __device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uin
 #pragma unroll
         for (int r = 0; r < ITEMS; ++r)
             if (r < rounds && first + r * 32 < n) {
-                const unsigned d = static_cast<unsigned>(key[r] >> shift) & (RADIX - 1);
+                const unsigned d = static_cast<unsigned>(key[r] >> shift) & digit_mask;
                 const int pos = dbase[d] + mine[d] + rank[r];
                 skey[pos] = key[r];
                 sval[pos] = val[r];
@@ -848,9 +863,16 @@ constexpr int kMergeItems = 2;
 constexpr int kMergeTile = kMergeThreads * kMergeItems;
 constexpr int64_t kMergeMaxN = int64_t(1) << 20;
 
+template <typename KeyT>
+static inline KeyT merge_key_mask(int sort_bits)
+{
+    const int unused = 8 * static_cast<int>(sizeof(KeyT)) - sort_bits;
+    return static_cast<KeyT>(~KeyT(0)) >> unused;
+}
+
 // keys and positions of one tile of ids, sorted
 template <typename KeyT>
-__global__ void __launch_bounds__(kMergeThreads) merge_tile_kernel(const int64_t* __restrict__ ids, int64_t n, int key_bits,
+__global__ void __launch_bounds__(kMergeThreads) merge_tile_kernel(const int64_t* __restrict__ ids, int64_t n, int sort_bits,
                                                                    KeyT* __restrict__ keys, uint32_t* __restrict__ vals)
 {
     __shared__ KeyT skey[kMergeTile];
@@ -865,22 +887,23 @@ __global__ void __launch_bounds__(kMergeThreads) merge_tile_kernel(const int64_t
         sval[i] = static_cast<uint32_t>(tile0 + i);
     }
     __syncthreads();
-    block_sort_pairs<KeyT, kMergeThreads, kMergeItems>(skey, sval, wcnt, dbase, sm, count, key_bits);
+    block_sort_pairs<KeyT, kMergeThreads, kMergeItems>(skey, sval, wcnt, dbase, sm, count, sort_bits);
     for (int i = threadIdx.x; i < count; i += kMergeThreads) {
         keys[tile0 + i] = skey[i];
         vals[tile0 + i] = sval[i];
     }
 }
 
-// runs of `run` pairs (the last may be shorter) -> runs of 4 * run
+// runs of `run` pairs (the last may be shorter) -> runs of 4 * run.  `mask`: the key bits the tiles were sorted by.  The
+// ranks are a permutation only while the runs are in the order they are searched in.
 template <typename KeyT>
 __global__ void __launch_bounds__(256) merge_round_kernel(const KeyT* __restrict__ keys, const uint32_t* __restrict__ vals,
-                                                          int64_t n, int64_t run, KeyT* __restrict__ keys_out,
+                                                          int64_t n, int64_t run, KeyT mask, KeyT* __restrict__ keys_out,
                                                           uint32_t* __restrict__ vals_out)
 {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const KeyT key = keys[i];
+    const KeyT whole = keys[i], key = whole & mask;
     const uint32_t val = vals[i];
     const int64_t group0 = i / (4 * run) * (4 * run);
     const int own = static_cast<int>((i - group0) / run);
@@ -897,29 +920,34 @@ __global__ void __launch_bounds__(256) merge_round_kernel(const KeyT* __restrict
         for (int q = 0; q < 4; ++q) {
             if (lo[q] < hi[q]) {
                 const int64_t mid = (lo[q] + hi[q]) >> 1;
-                const KeyT other = keys[group0 + q * run + mid];
+                const KeyT other = keys[group0 + q * run + mid] & mask;
                 // equal keys of earlier runs come first
                 if (q < own ? other <= key : other < key) lo[q] = mid + 1; else hi[q] = mid;
             }
         }
     }
     const int64_t pos = group0 + lo[0] + lo[1] + lo[2] + lo[3];
-    keys_out[pos] = key;
+    keys_out[pos] = whole;
     vals_out[pos] = val;
 }
 
-// ids -> pairs sorted by the key bits [0, key_bits); result in the a-buffers (0) or the b-buffers (1).  n <= kMergeMaxN.
+#ifndef RECSDK_EMULATE
+// ids -> pairs sorted by the bits radix_sort_pairs sorts by; result in the a-buffers (0) or the b-buffers (1).
+// n <= kMergeMaxN.
 template <typename KeyT>
 static inline int merge_sort_ids(const int64_t* ids, int64_t n, int key_bits, KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b,
                                  uint32_t* vals_b, cudaStream_t st)
 {
-    merge_tile_kernel<KeyT><<<static_cast<unsigned>(ceil_div(n, kMergeTile)), kMergeThreads, 0, st>>>(ids, n, key_bits, keys_a,
+    const int sort_bits = radix_sorted_bits<KeyT>(key_bits);
+    const KeyT mask = merge_key_mask<KeyT>(sort_bits);
+    merge_tile_kernel<KeyT><<<static_cast<unsigned>(ceil_div(n, kMergeTile)), kMergeThreads, 0, st>>>(ids, n, sort_bits, keys_a,
                                                                                                     vals_a);
     int cur = 0;
     for (int64_t run = kMergeTile; run < n; run *= 4, cur ^= 1)
         merge_round_kernel<KeyT><<<static_cast<unsigned>(ceil_div(n, 256)), 256, 0, st>>>(
-            cur ? keys_b : keys_a, cur ? vals_b : vals_a, n, run, cur ? keys_a : keys_b, cur ? vals_a : vals_b);
+            cur ? keys_b : keys_a, cur ? vals_b : vals_a, n, run, mask, cur ? keys_a : keys_b, cur ? vals_a : vals_b);
     return cur;
 }
+#endif  // RECSDK_EMULATE
 
 }  // namespace recsdk

@@ -180,8 +180,8 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     p.long_list = ws.long_list;
     const int vec_per_row = (a->max_D + 3) / 4;
     if (do_plan && small) {
-        plan_small_kernel<KeyT><<<1, kSmallThreads, plan_small_smem<KeyT>(), st>>>(p, key_bits, ws.vals_a, ws.run_start,
-                                                                                  ws.counters, ws.meta, ws.desc);
+        plan_small_kernel<KeyT><<<1, kSmallThreads, plan_small_smem<KeyT>(), st>>>(
+            p, radix_sorted_bits<KeyT>(key_bits), ws.vals_a, ws.run_start, ws.counters, ws.meta, ws.desc);
     } else if (do_plan) {
         // The plan needs the indices and the LAYOUT of the gradient, not the gradient: it can run ahead, on
         // another stream, while the forward of the same batch (or the dense part) runs.

@@ -630,7 +630,7 @@ constexpr size_t plan_small_smem()
 }
 
 template <typename KeyT>
-__global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, int key_bits, uint32_t* __restrict__ vals_out,
+__global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, int sort_bits, uint32_t* __restrict__ vals_out,
                                                                    int* __restrict__ run_start, int64_t* counters,
                                                                    RunMeta* __restrict__ meta, int2* __restrict__ desc)
 {
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, 
             });
     }
     __syncthreads();
-    block_sort_pairs<KeyT, kSmallThreads, kSmallItems>(skey, sval, wcnt, srun, sm, n, key_bits);
+    block_sort_pairs<KeyT, kSmallThreads, kSmallItems>(skey, sval, wcnt, srun, sm, n, sort_bits);
     const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
     // run starts: each thread looks at `rounds` consecutive positions
     {

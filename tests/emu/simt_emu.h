@@ -23,6 +23,7 @@
 #define __restrict__
 #define __launch_bounds__(...)
 #define __align__(n) alignas(n)
+#define __shared__ static  // the blocks of a grid run one after the other
 struct float4 { float x, y, z, w; };
 struct int2 { int x, y; };
 struct alignas(16) int4 { int x, y, z, w; };
@@ -98,3 +99,43 @@ static inline T __shfl_sync(unsigned mask, T v, int src, int width = 32)
 }
 static inline int __all_sync(unsigned mask, int pred)
 { unsigned long long snap[32]; int all; collective(mask, 0, pred, 2, snap, &all); return all; }
+static inline int __popc(unsigned x) { return __builtin_popcount(x); }
+static inline void __syncwarp(unsigned mask = 0xffffffffu)
+{ unsigned long long snap[32]; int all; collective(mask, 0, 1, 3, snap, &all); }
+template <typename T>
+static inline unsigned __match_any_sync(unsigned mask, T v)
+{
+    unsigned long long snap[32]; int all;
+    collective(mask, static_cast<unsigned long long>(v), 1, 4, snap, &all);
+    unsigned peers = 0;
+    for (int i = 0; i < 32; ++i)
+        if (((mask >> i) & 1u) && snap[i] == static_cast<unsigned long long>(v)) peers |= 1u << i;
+    return peers;
+}
+template <typename T>
+static inline T __shfl_up_sync(unsigned mask, T v, int delta)
+{
+    unsigned long long raw = 0; memcpy(&raw, &v, sizeof(T));
+    unsigned long long snap[32]; int all;
+    collective(mask, raw, 1, 5, snap, &all);
+    const int lane = threadIdx.x & 31;
+    T out; memcpy(&out, &snap[lane >= delta ? lane - delta : lane], sizeof(T)); return out;
+}
+// ---- block barrier: all blockDim.x threads, with the "or" of a predicate
+static std::mutex g_bar_mu;
+static std::condition_variable g_bar_cv;
+static unsigned g_bar_arrived = 0, g_bar_generation = 0;
+static int g_bar_or = 0, g_bar_result = 0;
+static inline int __syncthreads_or(int pred)
+{
+    std::unique_lock<std::mutex> l(g_bar_mu);
+    const unsigned gen = g_bar_generation;
+    g_bar_or |= pred != 0;
+    if (++g_bar_arrived == blockDim.x) {
+        g_bar_result = g_bar_or; g_bar_or = 0; g_bar_arrived = 0; g_bar_generation++; g_bar_cv.notify_all();
+    } else if (!g_bar_cv.wait_for(l, std::chrono::seconds(30), [&] { return g_bar_generation != gen; })) {
+        fprintf(stderr, "EMU: block barrier timeout: thread %u\n", threadIdx.x); abort();
+    }
+    return g_bar_result;
+}
+static inline void __syncthreads() { __syncthreads_or(0); }

@@ -110,6 +110,20 @@ def test_unique_sizes(n, bits):
     np.testing.assert_array_equal(got.cpu().numpy(), inv)
 
 
+# ids wider than key_bits: every sort orders them by the same low bits, and the inverse names a place in the buffer
+@pytest.mark.parametrize("bits,wide", [(21, 31), (33, 44), (47, 63)])
+@pytest.mark.parametrize("n", [2_300, 70_001, (1 << 20) + 1])
+def test_unique_ids_wider_than_the_key(n, bits, wide):
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(n + bits)
+    ids = np.where(rng.random(n) < 0.7, rng.integers(0, 1 << wide, n), rng.integers(0, 40, n))
+    uq, got, cnt = ops.unique_sorted(_t(ids), bits)
+    u, inv = int(cnt.item()), got.cpu().numpy()
+    assert inv.min() >= 0 and inv.max() == u - 1 < n
+    np.testing.assert_array_equal(uq.cpu().numpy()[:u][inv], ids)
+
+
 # more tables than a group holds, empty segments, one mapper for two tables: as table after table
 @pytest.mark.parametrize("per_table", [[5], [0, 0], [0, 3000, 0, 1, 2049], [700] * 19 + [0, 4097]])
 @pytest.mark.parametrize("shared", [False, True])
