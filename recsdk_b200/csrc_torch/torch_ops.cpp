@@ -573,14 +573,17 @@ private:
         const int64_t* seg = off.data_ptr<int64_t>() + firstTable;
         std::vector<const recsdk_mapper_t*> ms(tables);
         std::vector<int64_t*> status(tables);
+        // a mapper that comes up again with a longer segment replaces its workspace: the older one is held until all
+        // tables are enqueued
+        std::vector<Tensor> held(tables);
         std::vector<void*> ws(tables);
         std::vector<size_t> ws_bytes(tables);
         for (int64_t t = 0; t < tables; ++t) {
-            const Tensor w = mappers[t]->workspace(seg[t + 1] - seg[t]);
+            held[t] = mappers[t]->workspace(seg[t + 1] - seg[t]);
             ms[t] = &mappers[t]->m_;
             status[t] = mappers[t]->status_.template data_ptr<int64_t>();
-            ws[t] = w.data_ptr();
-            ws_bytes[t] = w.numel();
+            ws[t] = held[t].data_ptr();
+            ws_bytes[t] = held[t].numel();
         }
         Tensor status_all = at::empty({(firstTable + tables) * RECSDK_STATUS_WORDS}, globalIds.options());
         check_rc(recsdk_mapper_unique_out_multi(ms.data(), tables, firstTable, globalIds.data_ptr<int64_t>(),

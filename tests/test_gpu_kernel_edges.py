@@ -169,6 +169,37 @@ def test_mappers_together_report_the_table_that_failed():
                                                   torch.zeros(4, dtype=torch.int64, device=DEV))
 
 
+# one mapper for several segments, each longer than the one before, so that its workspace grows while the call collects
+# the tables; the workspaces of the earlier segments have to outlive their kernels
+def test_registered_mapper_whose_workspace_grows_within_a_call():
+    from recsdk_b200 import IdsMapper, torch_ops
+
+    if not torch_ops.available():
+        pytest.skip("torch op library not built")
+    torch_ops.load()
+    per_table = [30, 700, 3_000, 9_000, 9_000, 40_000]
+    T, n = len(per_table), sum(per_table)
+    offs = torch.from_numpy(np.concatenate([[0], np.cumsum(per_table)]).astype(np.int64))
+    ids = _t(np.random.default_rng(5).integers(0, 30_000, n))
+    registered, other = torch.classes.recsdk.IdsMapper(65_536, True), torch.classes.recsdk.IdsMapper(65_536, True)
+    single, single_other = IdsMapper(65_536), IdsMapper(65_536)
+    outs = []
+    for way in (0, 1):
+        hi, uq, uid, inv = (torch.zeros(n, dtype=torch.int64, device=DEV) for _ in range(4))
+        uo = torch.zeros(T + 1, dtype=torch.int64, device=DEV)
+        if way == 0:
+            ms = [registered] * T
+            ms[4] = other
+            torch.classes.recsdk.IdsMapper.parallel_ids2indices_unique_out(ms, ids, hi, offs, uq, uid, inv, uo)
+        else:
+            for t in range(T):
+                (single_other if t == 4 else single).ids2indices_unique_out(ids, hi, offs, uq, uid, inv, uo, t)
+        outs.append([x.cpu().numpy() for x in (hi, uq, uid, inv, uo)])
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+    assert registered.size() == single.size() and other.size() == single_other.size()
+
+
 @pytest.mark.parametrize("D", [1, 6, 64, 132])
 @pytest.mark.parametrize("B,L", [(1, 1), (37, 7), (1_500, 33)])
 def test_jagged_dense_row_groups(B, L, D):
