@@ -861,7 +861,18 @@ __device__ __forceinline__ void block_sort_pairs(KeyT* skey, uint32_t* sval, uin
 constexpr int kMergeThreads = 1024;
 constexpr int kMergeItems = 2;
 constexpr int kMergeTile = kMergeThreads * kMergeItems;
-constexpr int64_t kMergeMaxN = int64_t(1) << 20;
+
+// Where it is the faster one: its rounds grow with n (every pair searches three runs), the radix sort's passes with the
+// bits.  Sorted unique of uniform ids, radix / merge in us: 65536 ids of 21 bits (3 passes) 55.5 / 51.5, 98304 57.6 / 55.6,
+// 131072 57 / 64; of 32 bits (4) at 98304 74 / 60, at 196608 76 / 88; of 48 bits (5) at 131072 113 / 83, at 262144
+// 117 / 127; of 56 bits (6) at 196608 135 / 111, at 262144 135 / 132; of 62 bits (7) at 196608 152 / 114, at 524288
+// 201 / 225.  Equal ids leave the radix sort's stores in order and move the borders down a little.
+static inline bool merge_sort_pays(int64_t n, int key_bits)
+{
+    int passes, bits;
+    radix_plan(key_bits, &passes, &bits);
+    return n > 1 && passes >= 3 && n <= 32768 * (passes - 1);
+}
 
 template <typename KeyT>
 static inline KeyT merge_key_mask(int sort_bits)
@@ -933,7 +944,6 @@ __global__ void __launch_bounds__(256) merge_round_kernel(const KeyT* __restrict
 
 #ifndef RECSDK_EMULATE
 // ids -> pairs sorted by the bits radix_sort_pairs sorts by; result in the a-buffers (0) or the b-buffers (1).
-// n <= kMergeMaxN.
 template <typename KeyT>
 static inline int merge_sort_ids(const int64_t* ids, int64_t n, int key_bits, KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b,
                                  uint32_t* vals_b, cudaStream_t st)

@@ -58,11 +58,6 @@ static UniqueWorkspace carve_unique(void* base, int64_t N)
     return w;
 }
 
-// Keys wider than this take the merge sort (up to its size limit): its rounds depend on n alone, the radix sort's passes
-// on the bits.  131072 keys: 25 launches with 152 us in them by seven radix passes of
-// 10 bits, 6 launches merged, and the cached-table step around them 1.0 -> 0.85 ms; up to 20 bits are two passes.
-constexpr int kMergeMinBits = 20;
-
 template <typename KeyT>
 static int run_unique(const int64_t* ids, int64_t n, int key_bits, int64_t* unique_out, int64_t* inverse_out,
                       int64_t* num_unique_out, const UniqueWorkspace& ws, cudaStream_t st)
@@ -70,7 +65,7 @@ static int run_unique(const int64_t* ids, int64_t n, int key_bits, int64_t* uniq
     KeyT* ka = static_cast<KeyT*>(ws.keys_a);
     KeyT* kb = static_cast<KeyT*>(ws.keys_b);
     int which;
-    if (key_bits > kMergeMinBits && n <= kMergeMaxN) {
+    if (merge_sort_pays(n, key_bits)) {
         which = merge_sort_ids<KeyT>(ids, n, key_bits, ka, ws.vals_a, kb, ws.vals_b, st);
     } else {
         unique_load_kernel<KeyT><<<grid_for(n, 256), 256, 0, st>>>(ids, n, ka, ws.vals_a);

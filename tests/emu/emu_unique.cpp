@@ -45,3 +45,5 @@ extern "C" void emu_merge_sort(const int64_t* ids, int64_t n, int key_bits, uint
     if (key_bits <= 32) sort_ids<uint32_t>(ids, n, key_bits, order);
     else sort_ids<uint64_t>(ids, n, key_bits, order);
 }
+
+extern "C" int emu_merge_sort_pays(int64_t n, int key_bits) { return merge_sort_pays(n, key_bits) ? 1 : 0; }

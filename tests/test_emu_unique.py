@@ -25,7 +25,18 @@ def emu():
     lib = C.CDLL(OUT)
     lib.emu_merge_sort.restype = None
     lib.emu_merge_sort.argtypes = [C.c_void_p, C.c_int64, C.c_int, C.c_void_p]
+    lib.emu_merge_sort_pays.restype = C.c_int
+    lib.emu_merge_sort_pays.argtypes = [C.c_int64, C.c_int]
     return lib
+
+
+# sizes at which one of the two sorts took at least a tenth less time than the other
+@pytest.mark.parametrize("n,key_bits,merge", [
+    (1, 64, 0), (2_048, 20, 0), (2_048, 21, 1), (32_768, 21, 1), (131_072, 21, 0), (196_608, 32, 0), (98_304, 32, 1),
+    (131_072, 48, 1), (262_144, 40, 0), (196_608, 64, 1), (131_072, 62, 1), (262_144, 30, 0),
+    (524_288, 64, 0), (1 << 20, 21, 0), (1 << 20, 64, 0)])
+def test_the_faster_sort_is_taken(emu, n, key_bits, merge):
+    assert emu.emu_merge_sort_pays(n, key_bits) == merge
 
 
 def sorted_bits(key_bits):

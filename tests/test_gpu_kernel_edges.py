@@ -93,9 +93,11 @@ def test_bucketize_dedup(features, batch, max_len, vocab, world):
             np.testing.assert_array_equal(cnt.cpu().numpy()[:k], ec)
 
 
-# tiles of 2048, rounds of four runs, the size limit of the merge sort; the widths on either side of its rule
+# tiles of 2048, rounds of four runs, the size limits of the merge sort (65536 for 21 bits, 98304 for 33, 196608 for 64)
+# and where the sort for large inputs begins; the widths on either side of its rule
 @pytest.mark.parametrize("bits", [20, 21, 33, 64])
-@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 8193, 40_000, (1 << 20) + 1])
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 8193, 40_000, 65_536, 65_537, 98_304, 98_305, 131_073, 196_608, 196_609,
+                               (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
 def test_unique_sizes(n, bits):
     from recsdk_b200 import ops
 
