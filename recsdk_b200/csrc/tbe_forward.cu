@@ -207,8 +207,8 @@ __device__ __forceinline__ void pooled_walk(const FwdParams& p, const BagLane& b
     }
 }
 
-// Latency decides wherever the bags do not fill the chip, so a group takes as many bags (p.bags_per_group <= G) as
-// leave every SM several waves of groups; see bags_per_group().
+// Latency decides wherever the bags do not fill the chip, so a group takes only as many bags (p.bags_per_group <= G) as
+// pooled_plan() says.
 template <int G, int K, bool LONG = false>
 __global__ void __launch_bounds__(256, K == 4 ? 3 : 4) tbe_forward_pooled_kernel(FwdParams p)
 {
@@ -279,29 +279,46 @@ __global__ void __launch_bounds__(256) tbe_forward_nobag_kernel(FwdParams p)
     }
 }
 
-#ifndef RECSDK_EMULATE  // host side: not part of host-side SIMT emulation builds (tests/emu)
-// Bags per group: a power of two, G (coalesced metadata, one lane per bag) only while that still leaves four waves of
-// resident groups (1024 threads per SM at 64 registers).  With G always: 962 bags of up to 10 rows of 128 floats were
-// 30 warps on 148 SMs and took 29.5 us, now 4.1; 98304 bags of up to 30 rows of 256 floats were 0.65 waves, 231 us,
-// now 174 (161 with the bag-by-bag walk).  (Two waves instead of four: 177 against 174 us there.)
-static int bags_per_group(int64_t num_bags, int G)
+// How the pooled kernel goes about a batch: bags per group (a power of two up to G) and the walk.
+//
+// Bags per group: G keeps the metadata coalesced, one lane per bag, but must leave enough groups to fill the chip
+// (1024 threads per SM, 768 for the widest rows).  Rows of up to 32 floats and bags of less than four ids are content with
+// 5/8 of a wave; wider rows want two waves, and the bag-by-bag walk of rows of 128 floats and more four, for its uneven
+// bags.
+// With G always: 962 bags of up to 10 rows of 128 floats were 30 warps on 148 SMs, 29.5 us, now 4.1; 98304 bags of up to
+// 30 rows of 256 floats 231 us, now 161 (169 with two waves, 202 with one).  100000 bags of one id, 32 floats: 14.6 us
+// with eight bags per group, 18.9 with one; 400000 bags of 16 ids, 8 floats: 230 us with two, 286 with one.
+//
+// Walk: the bag-by-bag walk saves instructions per row, which counts from about eight ids per bag, two of its steps (a
+// training step of 20 M ids in bags of 50 2984 -> 2970 us, 98304 bags of 15.5 rows of 256 floats 177 -> 164).  It walks at
+// most G rows at a time, though: rows of 8 and 16 floats (G 2, 4) are 8 to 20 % slower by it at any size, and rows of 32
+// and 64 as soon as a group holds several bags (400000 bags of 12 ids, 32 floats: 168 against 192 us), unless the bags
+// are long (100000 of 50 ids, 64 floats: 294 against 263).  G == 1 has no rows to share: 148 against 80 us.
+struct PooledPlan {
+    int bags_per_group;
+    bool bag_by_bag;
+};
+static PooledPlan pooled_plan(int64_t num_bags, int64_t num_ids, int G, int K)
 {
-    const int64_t four_waves = static_cast<int64_t>(num_sms()) * (1024 / G) * 4;
-    int per = 1;
-    while (per < G && static_cast<int64_t>(per) * 2 * four_waves <= num_bags) per <<= 1;
-    return per;
+    const int64_t wave = static_cast<int64_t>(num_sms()) * ((K == 4 ? 768 : 1024) / G);
+    const bool long_bags = num_ids >= 8 * num_bags;
+    const int64_t eighths = (G <= 8 || num_ids < 4 * num_bags) ? 5 : (G == 32 && long_bags ? 32 : 16);
+    PooledPlan pl;
+    pl.bags_per_group = 1;
+    while (pl.bags_per_group < G && pl.bags_per_group * 2 * wave * eighths <= 8 * num_bags) pl.bags_per_group <<= 1;
+    if (G == 1 || G == 32) pl.bag_by_bag = long_bags;
+    else if (G >= 8 && pl.bags_per_group <= 2) pl.bag_by_bag = long_bags;
+    else pl.bag_by_bag = G == 16 && num_ids >= 32 * num_bags;
+    return pl;
 }
 
-// Ids per bag, on average, from which the bag-by-bag walk takes over: 98304 bags of
-// 15.5 rows of 256 floats 174 -> 161 us, a training step of 20 M ids in bags of 50 2984 -> 2970 us.  Bags of one or two ids
-// need the other walk to have several rows in flight; eight are two of its steps.
-constexpr int64_t kLongBagIds = 8;
-
+#ifndef RECSDK_EMULATE  // launches: not part of host-side SIMT emulation builds (tests/emu)
 template <int G, int K>
 static void launch_pooled(FwdParams p, bool leave_room, cudaStream_t st)
 {
     const int groups_per_block = 256 / G;
-    p.bags_per_group = bags_per_group(p.T * p.B, G);
+    const PooledPlan plan = pooled_plan(p.T * p.B, p.N, G, K);
+    p.bags_per_group = plan.bags_per_group;
     // several waves of short-lived blocks rather than one resident wave: when the backward's index kernels run
     // beside this one on another stream, their blocks get SM slots as these retire (measured: 16 per SM 0.833 ms
     // per benchmark step, 8: 0.838, 2: 0.873; alone the grid size makes no difference)
@@ -312,9 +329,15 @@ static void launch_pooled(FwdParams p, bool leave_room, cudaStream_t st)
         if (leave_room && smem_optin(kernel, 60 * 1024, optin_done)) smem = 60 * 1024;
         kernel<<<grid, 256, smem, st>>>(p);
     };
-    static bool optin_short[kMaxDevices] = {false}, optin_long[kMaxDevices] = {false};
-    if (p.N >= kLongBagIds * p.T * p.B) launch(tbe_forward_pooled_kernel<G, K, true>, optin_long);
-    else launch(tbe_forward_pooled_kernel<G, K, false>, optin_short);
+    static bool optin_short[kMaxDevices] = {false};
+    if constexpr (G != 2 && G != 4) {  // see pooled_plan()
+        static bool optin_long[kMaxDevices] = {false};
+        if (plan.bag_by_bag) {
+            launch(tbe_forward_pooled_kernel<G, K, true>, optin_long);
+            return;
+        }
+    }
+    launch(tbe_forward_pooled_kernel<G, K, false>, optin_short);
 }
 
 template <int G>

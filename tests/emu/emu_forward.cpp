@@ -44,3 +44,10 @@ extern "C" int emu_tbe_forward_pooled(const float* w, const int64_t* wofs, const
 #undef RUN
     return 1;
 }
+
+// bags per group, + 100 for the bag-by-bag walk
+extern "C" int emu_pooled_plan(int64_t num_bags, int64_t num_ids, int G, int K)
+{
+    const PooledPlan pl = pooled_plan(num_bags, num_ids, G, K);
+    return pl.bags_per_group + (pl.bag_by_bag ? 100 : 0);
+}
