@@ -282,12 +282,13 @@ __global__ void __launch_bounds__(256) tbe_forward_nobag_kernel(FwdParams p)
 // How the pooled kernel goes about a batch: bags per group (a power of two up to G) and the walk.
 //
 // Bags per group: G keeps the metadata coalesced, one lane per bag, but must leave enough groups to fill the chip
-// (1024 threads per SM, 768 for the widest rows).  Rows of up to 32 floats and bags of less than four ids are content with
-// 5/8 of a wave; wider rows want two waves, and the bag-by-bag walk of rows of 128 floats and more four, for its uneven
-// bags.
+// (1024 threads per SM, 768 for the widest rows).  Rows of up to 32 floats, and of up to 128 in bags of less than four
+// ids, are content with 5/8 of a wave; wider rows want two waves, and the bag-by-bag walk of rows of 128 floats and more
+// four, for its uneven bags.
 // With G always: 962 bags of up to 10 rows of 128 floats were 30 warps on 148 SMs, 29.5 us, now 4.1; 98304 bags of up to
 // 30 rows of 256 floats 231 us, now 161 (169 with two waves, 202 with one).  100000 bags of one id, 32 floats: 14.6 us
-// with eight bags per group, 18.9 with one; 400000 bags of 16 ids, 8 floats: 230 us with two, 286 with one.
+// with eight bags per group, 18.9 with one; 100000 bags of four, 256 floats: 77 us with 32, 66 with eight; 400000 bags
+// of 16 ids, 8 floats: 230 us with two, 286 with one.
 //
 // Walk: the bag-by-bag walk saves instructions per row, which counts from about eight ids per bag, two of its steps (a
 // training step of 20 M ids in bags of 50 2984 -> 2970 us, 98304 bags of 15.5 rows of 256 floats 177 -> 164).  It walks at
@@ -302,7 +303,7 @@ static PooledPlan pooled_plan(int64_t num_bags, int64_t num_ids, int G, int K)
 {
     const int64_t wave = static_cast<int64_t>(num_sms()) * ((K == 4 ? 768 : 1024) / G);
     const bool long_bags = num_ids >= 8 * num_bags;
-    const int64_t eighths = (G <= 8 || num_ids < 4 * num_bags) ? 5 : (G == 32 && long_bags ? 32 : 16);
+    const int64_t eighths = (G <= 8 || (K == 1 && num_ids < 4 * num_bags)) ? 5 : (G == 32 && long_bags ? 32 : 16);
     PooledPlan pl;
     pl.bags_per_group = 1;
     while (pl.bags_per_group < G && pl.bags_per_group * 2 * wave * eighths <= 8 * num_bags) pl.bags_per_group <<= 1;

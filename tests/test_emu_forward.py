@@ -40,7 +40,8 @@ def emu():
 
 # measured: the walk, and whole groups, that took less time at these sizes (148 SMs)
 @pytest.mark.parametrize("bags,ids_per_bag,G,K,per,bag_by_bag", [
-    (500, 40, 32, 1, 1, True), (98_304, 15.5, 32, 2, 4, True), (400_000, 1, 32, 1, 32, False),
+    (500, 40, 32, 1, 1, True), (98_304, 15.5, 32, 2, 4, True), (400_000, 1, 32, 1, 32, False), (100_000, 3.9, 32, 2, 8, False),
+    (100_000, 1, 32, 1, 32, False),
     (400_000, 16, 2, 1, 2, False), (100_000, 40, 2, 1, 2, False), (100_000, 40, 4, 1, 4, False), (20_000, 50, 2, 1, 1, False),
     (100_000, 1, 8, 1, 8, False), (400_000, 12, 8, 1, 8, False), (20_000, 8, 8, 1, 1, True),
     (400_000, 8, 16, 1, 16, False), (50_000, 12, 16, 1, 2, True), (425_984, 50, 16, 1, 16, True), (100_000, 8, 1, 1, 1, True)])
