@@ -617,8 +617,10 @@ __global__ void __launch_bounds__(256) run_meta_kernel(BwdParams p, const KeyT* 
 // ---------------------------------------------------------------------------- 1.-4. the whole plan of a small batch
 // One block does what expand, the sort passes, the run scan and the records do for a batch that fits its shared memory
 // (at most kSmallN positions in at most kSmallN bags).  Such a batch is bound by launches and by the latency of each
-// kernel's first loads, not by work: 4096 ids of 20-bit keys took eleven launches, 37 us of kernels and the gaps between them, against 25 us
-// in this one launch (a training step of them 116 -> 93..102 us).  
+// kernel's first loads, not by work.  Uniform ids, the launches / this one, replayed from a graph: 4096 of 20 bits
+// 42 / 31 us, 8192 of 40 bits 64 / 58; 8192 of 20 to 27 bits 45 / 51, where one block has become the slower one on the
+// device.  The border stays at what shared memory holds all the same: the eleven launches cost the host more than that
+// (training step of 4096 ids 125 -> 98 us, of 8192 ids 124 -> 99).
 constexpr int kSmallN = 8192;
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallItems = kSmallN / kSmallThreads;
