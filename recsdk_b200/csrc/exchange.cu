@@ -461,7 +461,7 @@ static XchgWorkspace carve_xchg(void* base, int64_t max_ids, int64_t inbox_cap, 
     WorkspaceCarver c(base);
     XchgWorkspace w;
     const size_t n = static_cast<size_t>(max_ids > 0 ? max_ids : 1);
-    const size_t chunks = chunk_slots_cap(max_ids);
+    const size_t chunks = chunk_slots(max_ids, kDirectMax);  // both phases keep this threshold
     w.lc = c.take<int64_t>(8);
     w.seg = c.take<int64_t>(RECSDK_MAX_SHARDS + 1);
     w.keys_a = c.take<uint64_t>(n);
@@ -484,7 +484,7 @@ static XchgWorkspace carve_xchg(void* base, int64_t max_ids, int64_t inbox_cap, 
     w.fetched = c.take<float>(n * static_cast<size_t>(D));
     const int64_t in_cap = static_cast<int64_t>(world) * inbox_cap;
     const size_t m = static_cast<size_t>(in_cap > 0 ? in_cap : 1);
-    const size_t ochunks = chunk_slots_cap(in_cap);
+    const size_t ochunks = chunk_slots(in_cap, kDirectMax);
     w.oc = c.take<int64_t>(8);
     w.lay_i64 = c.take<int64_t>(4);
     w.lay_i32 = c.take<int32_t>(4);
@@ -702,7 +702,8 @@ static int xchg_forward_impl(const recsdk_xchg_t* x, const XchgWorkspace& ws, co
 template <int G, int K>
 static void xchg_launch_partial(const BwdParams& p, int64_t n, cudaStream_t st)
 {
-    partial_kernel<G, K><<<grid_for(static_cast<int64_t>(chunk_slots_cap(n)), 256 / G, 4 * chunk_blocks(G)), 256, 0, st>>>(p);
+    const int64_t slots = static_cast<int64_t>(chunk_slots(n, p.direct_max));
+    partial_kernel<G, K><<<grid_for(slots, 256 / G, 4 * chunk_blocks(G)), 256, 0, st>>>(p);
 }
 
 template <int G, int K>

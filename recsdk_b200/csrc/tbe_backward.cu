@@ -126,7 +126,7 @@ static void launch_partial(const BwdParams& p, int64_t N, cudaStream_t st)
     const int groups_per_block = 256 / G;
     // four waves of resident blocks: how many chunks there are is known on the device only, and a grid that is no
     // multiple of the resident blocks leaves SMs idle behind the last wave
-    const int grid = grid_for(static_cast<int64_t>(chunk_slots_cap(N)), groups_per_block, 4 * chunk_blocks(G));
+    const int grid = grid_for(static_cast<int64_t>(chunk_slots(N, p.direct_max)), groups_per_block, 4 * chunk_blocks(G));
     partial_kernel<G, K><<<grid, 256, 0, st>>>(p);
 }
 

@@ -53,14 +53,17 @@ constexpr int kDirectMax = kChunk;
 constexpr int kDirectMaxSmall = 8;
 constexpr int64_t kDirectSmallN = int64_t(1) << 20;
 static inline int direct_max_for(int64_t n) { return n <= kDirectSmallN ? kDirectMaxSmall : kDirectMax; }
-// Slots of the partial buffer / chunk descriptors that n index positions, or any smaller number of them, can need (a
-// workspace sized for the largest batch serves every smaller one).
-static inline size_t chunk_slots_cap(int64_t n)
+// Slots of the partial buffer / chunk descriptors that n index positions can need with one threshold for direct runs.
+static inline size_t chunk_slots(int64_t n, int direct_max)
 {
     const size_t m = static_cast<size_t>(n > 0 ? n : 1);
-    const size_t few = m < static_cast<size_t>(kDirectSmallN) ? m : static_cast<size_t>(kDirectSmallN);
-    const size_t small = few / kChunk + few / (kDirectMaxSmall + 1), large = m / kChunk + m / (kDirectMax + 1);
-    return (small > large ? small : large) + 2;
+    return m / kChunk + m / (direct_max + 1) + 2;
+}
+// The same for any number of them up to n (a workspace sized for the largest batch serves every smaller one).
+static inline size_t chunk_slots_cap(int64_t n)
+{
+    const size_t small = chunk_slots(n < kDirectSmallN ? n : kDirectSmallN, kDirectMaxSmall), large = chunk_slots(n, kDirectMax);
+    return small > large ? small : large;
 }
 // Above this many chunks the sum over a run's chunk sums gets a kernel of its own (long_run_kernel).  The order of that
 // sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update keeps four in flight

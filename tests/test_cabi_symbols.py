@@ -44,6 +44,18 @@ def test_host_only_entry_points():
     assert lib.recsdk_unique_sorted(None, -1, 64, None, None, None, None, 0, None) == _lib.ERR_INVALID_ARG
 
 
+def test_exchange_workspace_holds_the_chunk_sums_it_can_make():
+    """Runs of up to 64 positions are summed without a slot in both phases, so n ids need at most n / 64 + n / 65 slots."""
+    from recsdk_b200 import _lib
+
+    lib = _lib.load()
+    n, inbox, world = 1 << 20, 1 << 18, 2
+    wide, narrow = (lib.recsdk_xchg_workspace_bytes(n, inbox, world, d, 3) for d in (320, 64))
+    rows = (wide - narrow) // (256 * 4)  # rows of D floats: one per id, and the slots
+    slots = sum(m // 64 + m // 65 + 2 for m in (n, world * inbox))
+    assert abs(rows - (n + slots)) <= 2
+
+
 def test_cpu_tensors_are_rejected():
     import torch
     from recsdk_b200 import ops
