@@ -41,18 +41,18 @@ namespace recsdk {
 
 constexpr int kChunk = 64;  // the only non-zero reduce_chunk supported
 // Runs of more than direct_max positions are summed by the chunk-sum kernel (lanes resolve the gradient rows of a
-// chunk in parallel and keep eight or more row loads in flight), the row-update kernel then reads one partial row per
-// chunk; shorter runs are summed inside the row-update kernel, four rows at a time.  This routing does not touch the
+// chunk in parallel and keep chunk_loads(G) / K row loads in flight), the row-update kernel then reads one partial row
+// per chunk; shorter runs are summed inside the row-update kernel, four rows at a time.  This routing does not touch the
 // arithmetic: a run of at most reduce_chunk positions is ONE chunk, and 0.0f + (its sequential sum) is that sum bit for
 // bit (with reduce_chunk 0 a longer run is one chunk as a whole).
-// Large batches hide the row update's chain behind other rows: thresholds 8, 16, 32 and 64 are within 2 % of each
-// other on the benchmark step, and 64 needs the smallest partial buffer.  Below kDirectSmallN ids the chain of the
-// longest direct run is what the kernel takes: 11 tables of 8..128 floats, 330 K ids, MEAN: 70 us with 64,
-// 47 with 8 (and the chunk sums 15 and 24).
+// Small batches take as long as the chain of the longest direct run, large ones hide it behind other rows and pay for
+// every slot.  Chunk sums and row update together, us, with thresholds 8 / 16 / 64: 32768 log-uniform ids over 400000
+// rows of 8 floats 29 / 31 / 37; 131072 of 32 floats 37 / 37 / 41; training steps of 11 tables, 330 K ids, MEAN 202 / 198 /
+// 210 and of 205 K ids unpooled 235 / 235 / 243; 524288 uniform ids of 32 floats 80 / 74 / 75; 2^20 of 128 floats 308 / 303 /
+// 303, and the plan of 2^20 log-uniform ids 98 / 90 / 82.
 constexpr int kDirectMax = kChunk;
-constexpr int kDirectMaxSmall = 8;
-constexpr int64_t kDirectSmallN = int64_t(1) << 20;
-static inline int direct_max_for(int64_t n) { return n <= kDirectSmallN ? kDirectMaxSmall : kDirectMax; }
+constexpr int64_t kDirect8N = int64_t(1) << 17, kDirect16N = int64_t(1) << 19;
+static inline int direct_max_for(int64_t n) { return n <= kDirect8N ? 8 : (n <= kDirect16N ? 16 : kDirectMax); }
 // Slots of the partial buffer / chunk descriptors that n index positions can need with one threshold for direct runs.
 static inline size_t chunk_slots(int64_t n, int direct_max)
 {
@@ -62,8 +62,13 @@ static inline size_t chunk_slots(int64_t n, int direct_max)
 // The same for any number of them up to n (a workspace sized for the largest batch serves every smaller one).
 static inline size_t chunk_slots_cap(int64_t n)
 {
-    const size_t small = chunk_slots(n < kDirectSmallN ? n : kDirectSmallN, kDirectMaxSmall), large = chunk_slots(n, kDirectMax);
-    return small > large ? small : large;
+    size_t most = chunk_slots(n, kDirectMax);
+    for (int64_t border : {kDirect8N, kDirect16N}) {
+        const int64_t m = n < border ? n : border;
+        const size_t slots = chunk_slots(m, direct_max_for(m));
+        most = slots > most ? slots : most;
+    }
+    return most;
 }
 // Above this many chunks the sum over a run's chunk sums gets a kernel of its own (long_run_kernel).  The order of that
 // sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update keeps four in flight
@@ -109,7 +114,7 @@ struct BwdParams {
     // kOptStore only (the dedup exchange's local phase): where the per-row sums go.  A record's row_off is then
     // (buffer number << kLocShardShift) | element offset inside that buffer; the buffers may be peer mappings.
     float* dst_ptrs[RECSDK_MAX_SHARDS];
-    int32_t direct_max;  // runs longer than this go through the chunk-sum kernel (>= kDirectMax)
+    int32_t direct_max;  // runs longer than this go through the chunk-sum kernel
     // > 0: runs of more than this many chunks are listed in long_list (counters[4] of them) and long_run_kernel leaves
     // their total in their first chunk slot before the row update reads it
     int32_t long_chunks;
@@ -558,14 +563,13 @@ struct __align__(16) RunMeta {
     int64_t g0_loc;      // location (grad_row_loc) of the run's first gradient row
     int32_t rs, len;     // sorted positions [rs, rs + len)
     int32_t D;           // row width in elements; kMetaVecBit set when the 128-bit path applies
-    int32_t chunk_base;  // first slot of the run in the partial buffer (len > kChunk), else -1
+    int32_t chunk_base;  // first slot of the run in the partial buffer (len > direct_max), else -1
 };
 constexpr int32_t kMetaVecBit = 1 << 30;
 
-// A run longer than kDirectMax also reserves its chunk slots in the partial buffer -- ceil(len/reduce_chunk), or one
-// for the whole run when reduce_chunk is 0 -- (atomic
-// counter; slot numbers differ from launch to launch but a slot's content and the order in which
-// a run's slots are summed do not) and describes each chunk as [begin, end) in sorted positions.
+// A run longer than p.direct_max also reserves its chunk slots in the partial buffer -- ceil(len/reduce_chunk), or one
+// for the whole run when reduce_chunk is 0 -- (atomic counter; slot numbers differ from launch to launch but a slot's
+// content and the order in which a run's slots are summed do not) and describes each chunk as [begin, end) in sorted positions.
 // counters[2] collects how many indices live in chunked runs (bandwidth accounting only).
 __device__ __forceinline__ RunMeta make_run_meta(const BwdParams& p, int64_t r, int rs, int re, int64_t key, uint32_t v0,
                                                  bool unaligned_cols, int64_t* __restrict__ counters, int2* __restrict__ desc)

@@ -94,3 +94,6 @@ extern "C" int emu_tbe_backward(const float* grad, float* w, float* m1, float* m
     free(partial);
     return rc;
 }
+
+extern "C" int emu_direct_max(int64_t n) { return direct_max_for(n); }
+extern "C" int64_t emu_chunk_slots_cap(int64_t n) { return static_cast<int64_t>(chunk_slots_cap(n)); }

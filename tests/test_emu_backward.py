@@ -30,7 +30,24 @@ def emu():
     lib.emu_tbe_backward.restype = C.c_int
     lib.emu_tbe_backward.argtypes = [vp] * 9 + [C.c_int64] * 3 + [C.c_int32] * 5 + [C.c_float] * 5 + [C.c_int64, vp] + \
         [C.c_int] * 4
+    lib.emu_direct_max.restype = C.c_int
+    lib.emu_direct_max.argtypes = [C.c_int64]
+    lib.emu_chunk_slots_cap.restype = C.c_int64
+    lib.emu_chunk_slots_cap.argtypes = [C.c_int64]
     return lib
+
+
+# measured: the threshold for direct runs that took the least time, plan included
+@pytest.mark.parametrize("n,threshold", [(8_192, 8), (131_072, 8), (330_000, 16), (524_288, 16), (1 << 20, 64), (1 << 21, 64)])
+def test_direct_run_threshold(emu, n, threshold):
+    assert emu.emu_direct_max(n) == threshold
+
+
+def test_chunk_slots_serve_every_smaller_batch(emu):
+    sizes = sorted({max(1, (1 << k) + d) for k in range(0, 24) for d in (-1, 0, 1)} | {330_000, 700_000})
+    need = [max(m // 64 + m // (emu.emu_direct_max(m) + 1) for m in sizes if m <= n) for n in sizes]
+    assert all(emu.emu_chunk_slots_cap(n) >= k for n, k in zip(sizes, need))
+    assert emu.emu_chunk_slots_cap(1 << 20) <= (1 << 20) // 24  # one threshold of 8 up to 2^20 ids: 133 K slots
 
 
 def _ptr(a):
