@@ -175,8 +175,8 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     p.counters = ws.counters;
     p.chunk_desc = ws.desc;
     p.partial = ws.partial;
-    // below this many ids even one row that holds them all has a chain of a few dozen rounds: not worth a launch
-    p.long_chunks = (N >= kLongRunMinIds && p.chunk > 0) ? kLongChunks : 0;
+    // below this many ids hardly any row is that long and the launch costs more than its chain
+    p.long_runs = (N >= kLongRunMinIds && p.chunk > 0) ? 1 : 0;
     p.long_list = ws.long_list;
     const int vec_per_row = (a->max_D + 3) / 4;
     if (do_plan && small) {
@@ -216,7 +216,11 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
 #undef CALL_PARTIAL
     }
     // 4c. totals of the runs with many chunks
-    if (p.long_chunks > 0) long_run_kernel<<<num_sms() * 6, kLongWarps * 32, 0, st>>>(p, ws.meta);
+    if (p.long_runs != 0) {
+        // one warp per run and 32 columns, as far as there can be any
+        const int64_t items = static_cast<int64_t>(long_runs_cap(N)) * ((p.max_D + 31) / 32);
+        long_run_kernel<<<grid_for(items, kLongWarps, 6), kLongWarps * 32, 0, st>>>(p, ws.meta);
+    }
     // 5. update
     if (a->ev_update_start) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_update_start), st);
 #define CALL_UPDATE(G, K) launch_update<G, K>(p, ws.meta, N, st)

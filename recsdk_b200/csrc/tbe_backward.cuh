@@ -70,11 +70,20 @@ static inline size_t chunk_slots_cap(int64_t n)
     }
     return most;
 }
-// Above this many chunks the sum over a run's chunk sums gets a kernel of its own (long_run_kernel).  The order of that
-// sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update keeps four in flight
-// beside its table row, a warp of that kernel 224.  Hottest row of 20 M Zipf(1.2) ids in 26 tables, about 2600 chunks:
-// the row update as a whole took 1027 us with its chain in it, 724 without, and this kernel 60.
-constexpr int kLongChunks = 64;
+// The sum over the chunk sums of a hot row gets a kernel of its own (long_run_kernel) where the row update would wait for
+// it.  The order of that sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update
+// keeps four in flight beside its table row, a warp of that kernel 224.  Hottest row of 20 M Zipf(1.2) ids in 26 tables,
+// about 2600 chunks: the row update as a whole took 1027 us with its chain in it, 724 without, and this kernel 60.
+// A chain of c chunks takes 0.15 to 0.4 us a chunk and is hidden while the update of all the other rows, about 1 to 1.6 us
+// per MB of them, takes longer: a run is listed for the kernel from kLongChunks + 4 per MB of updated rows on.
+// With every run above 64 chunks listed, chunk sums and update of 524288 log-uniform ids of 128 floats (64 MB of rows,
+// hottest row 440 chunks) took 122 us, with none 110; of 131072 ids of 64 floats 41 and 35; of 2^20 ids of 64 floats
+// (52 MB, 884 chunks) 139 and 180; of 65536 ids half of which are one row, 8 floats, 41 and 58.
+constexpr int kLongChunks = 224;
+__host__ __device__ __forceinline__ int64_t long_run_chunks(int64_t rows, int32_t max_D)
+{
+    return kLongChunks + ((rows * max_D) >> 18) * 4;
+}
 // Runs that can be longer than that: n positions hold at most n / (kLongChunks * kChunk) of them.
 static inline size_t long_runs_cap(int64_t n) { return static_cast<size_t>(n > 0 ? n : 0) / (kLongChunks * kChunk) + 1; }
 // Chunks of a run of `len` positions that went through the chunk-sum kernel.
@@ -115,11 +124,17 @@ struct BwdParams {
     // (buffer number << kLocShardShift) | element offset inside that buffer; the buffers may be peer mappings.
     float* dst_ptrs[RECSDK_MAX_SHARDS];
     int32_t direct_max;  // runs longer than this go through the chunk-sum kernel
-    // > 0: runs of more than this many chunks are listed in long_list (counters[4] of them) and long_run_kernel leaves
-    // their total in their first chunk slot before the row update reads it
-    int32_t long_chunks;
+    // != 0: runs of more than long_run_chunks() chunks are listed in long_list (counters[4] of them) and long_run_kernel
+    // leaves their total in their first chunk slot before the row update reads it
+    int32_t long_runs;
     int* __restrict__ long_list;
 };
+
+// Of a run of `chunks` chunks among `rows` distinct rows.
+__device__ __forceinline__ bool is_long_run(const BwdParams& p, int chunks, int64_t rows)
+{
+    return p.long_runs != 0 && chunks > kLongChunks && chunks > long_run_chunks(rows, p.max_D);
+}
 
 // Internal "optimizer" of the row-update kernels: no table is read, the summed gradient of the row is stored.
 constexpr int kOptStore = 0;
@@ -597,7 +612,7 @@ __device__ __forceinline__ RunMeta make_run_meta(const BwdParams& p, int64_t r, 
                                                     static_cast<unsigned long long>(c)));
         atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), static_cast<unsigned long long>(len));
         m.chunk_base = base;
-        if (p.long_chunks > 0 && c > p.long_chunks)
+        if (is_long_run(p, c, counters[0]))
             p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(counters + 4), 1ull)] = static_cast<int>(r);
         for (int k = 0; k < c; ++k) {
             const int b0 = rs + k * step;
@@ -710,7 +725,7 @@ __global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, 
     }
 }
 // ---------------------------------------------------------------------------- 4c. totals of the longest runs
-// One warp per (listed run, 32 columns): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
+// One warp per (listed run, see long_run_chunks(), 32 columns): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
 // place of the run's first chunk sum (no other warp reads these columns of this run).  The chunk sums come through a
 // ring of kLongStages shared-memory stages of 32 rows, filled by asynchronous copies, so 224 rows are in flight
 // whatever the registers; each lane copies and reads its own column, so a stage needs no barrier.
@@ -765,7 +780,7 @@ __device__ __forceinline__ void row_gradient(const BwdParams& p, const RunMeta& 
     const bool chunked = m.chunk_base >= 0;
     if (chunked) {
         int nc = chunks_of_run(m.len, p.chunk);
-        if (p.long_chunks > 0 && nc > p.long_chunks) nc = 1;  // long_run_kernel left the total in the first slot
+        if (is_long_run(p, nc, p.counters[0])) nc = 1;  // long_run_kernel left the total in the first slot
         int c = 0;
         for (; c + 4 <= nc; c += 4) {
             typename V::T v[4][K];

@@ -59,17 +59,49 @@ def test_backward_plan_sizes(n, bits):
     _backward_equals_oracle(rng.integers(0, 60_000, n), 60_000, 4, min(n, 5_000), bits)
 
 
-# runs around the direct / chunked border, a chunk, the border above which a run's chunk sums get their own kernel
+# runs around the direct / chunked borders (8, 16, 64 by the size of the batch), a chunk, the border above which a run's
+# chunk sums get their own kernel (224 chunks with so few rows), and that kernel's ring of 256 chunk sums taken around
+# more than once
+RUNS = [1, 2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 128, 129, 4095, 4096, 4097, 4161, 14_000, 16 * 64, 17 * 64 + 1]
+LONG_RUNS = [224 * 64, 224 * 64 + 1, 256 * 64, 256 * 64 + 1, 40_000]
+
+
 @pytest.mark.parametrize("dim", [4, 8, 16, 32, 36, 64, 128, 18])
 def test_backward_run_lengths(dim):
-    lengths = [1, 2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 128, 129, 4095, 4096, 4097, 4161, 14_000, 16 * 64, 17 * 64 + 1]
-    ids = np.repeat(np.arange(len(lengths)), lengths)
     rng = np.random.default_rng(dim)
-    rng.shuffle(ids)
-    assert ids.size > 32768  # the totals kernel runs
-    _backward_equals_oracle(ids, len(lengths), dim, 3_001, 8)
-    small = ids[ids < 12]
-    _backward_equals_oracle(small, len(lengths), dim, 301, 8, mode=1)
+
+    def check(lengths, bags, mode):
+        ids = rng.permutation(np.repeat(np.arange(len(lengths)), lengths))
+        _backward_equals_oracle(ids, len(lengths), dim, bags, 8, mode=mode)
+        return ids.size
+
+    assert check(RUNS[:12], 301, 1) < 8192
+    assert 32_768 < check(RUNS, 3_001, 0) < 1 << 17
+    assert 1 << 17 < check(RUNS + LONG_RUNS, 3_001, 0) < 1 << 19
+
+
+# the same kernel on rows narrower than the widest, their widths no multiple of its 32 columns
+@pytest.mark.parametrize("opt", [1, 2])
+@pytest.mark.parametrize("dims", [[20, 72], [100, 36], [7, 33]])
+def test_backward_long_runs_of_mixed_widths(dims, opt):
+    from recsdk_b200 import ops
+
+    rng = np.random.default_rng(sum(dims))
+    B, per_bag = 2_000, 16
+    n, total = 2 * B * per_bag, sum(dims)
+    indices = np.where(rng.random(n) < 0.9, 1, rng.integers(0, 3, n))
+    offsets = np.arange(2 * B + 1, dtype=np.int64) * per_bag
+    wo, do, hs = np.array([0, 3 * dims[0]], np.int64), np.array([0, dims[0], total], np.int32), np.array([0, 3, 6], np.int64)
+    grad = rng.standard_normal((B, total)).astype(np.float32)
+    w = rng.uniform(-0.05, 0.05, 3 * total).astype(np.float32)
+    m1, m2 = np.full_like(w, 0.1), np.full_like(w, 0.2)
+    dw, dm1, dm2 = _t(w), _t(m1), _t(m2)
+    port.tbe_backward(grad, w, m1, m2, wo, do, hs, indices, offsets, 2, B, total, max(dims), 0, opt, 0.05, 1e-8, 0.9, 0.999, 1,
+                      reduce_chunk=64)
+    ops.tbe_backward(_t(grad), dw, dm1, dm2, _t(wo), _t(do), _t(hs), _t(indices), _t(offsets), total, max(dims), 0, opt, 0.05,
+                     1e-8, 0.9, 0.999, 1, total_hash_size_bits=8, reduce_chunk=64)
+    for got, exp in ((dw, w), (dm1, m1), (dm2, m2)):
+        np.testing.assert_array_equal(got.cpu().numpy(), exp)
 
 
 @pytest.mark.parametrize("world", [1, 3, 64])
