@@ -390,8 +390,9 @@ static __global__ void __launch_bounds__(256) group_find_or_claim_kernel(const _
     const MapperSeg& s = g.seg[blockIdx.y];
     find_or_claim<0>(s.m.table, s.m.hash_capacity, s.ids, s.n, s.slots, s.ent, s.miss, nullptr, s.m.counters, s.status);
 }
-// Scan over one table's flags; tiles past the end of a short table have nothing to do.  The apply kernel adds up the
-// sums of the tiles before its own.
+// Scan over one table's flags; tiles past the end of a short table have nothing to do.  Up to kScanFoldTiles tiles the
+// apply kernel adds up the sums of the tiles before its own (`fold`); above, where that would be quadratic, one block per
+// table scans the sums in between.
 template <typename InFn>
 __device__ __forceinline__ void group_scan_reduce(const InFn& in, int64_t n, int* tile_sums)
 {
@@ -408,7 +409,7 @@ __device__ __forceinline__ void group_scan_reduce(const InFn& in, int64_t n, int
 }
 template <typename InFn, typename OutFn>
 __device__ __forceinline__ void group_scan_apply(const InFn& in, const OutFn& out, int64_t n, const int* tile_sums,
-                                                 int64_t* total_out)
+                                                 int fold, int64_t* total_out)
 {
     __shared__ int sm[33];
     if (static_cast<int64_t>(blockIdx.x) * kScanTile >= n) {
@@ -425,10 +426,7 @@ __device__ __forceinline__ void group_scan_apply(const InFn& in, const OutFn& ou
     }
     int total;
     const int inc = block_inclusive_scan(s, sm, &total);
-    int part = 0, before;
-    for (int t = threadIdx.x; t < static_cast<int>(blockIdx.x); t += blockDim.x) part += tile_sums[t];
-    block_inclusive_scan(part, sm, &before);
-    int run = before + inc - s;
+    int run = scan_tile_offset(tile_sums, fold, total, sm, nullptr) + inc - s;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < n) out(base + k, v[k], run, n);
@@ -436,16 +434,21 @@ __device__ __forceinline__ void group_scan_apply(const InFn& in, const OutFn& ou
     }
     if (base < n && base + kScanItems >= n) *total_out = run;  // the thread that holds the last item
 }
+static __global__ void __launch_bounds__(1024) group_tile_sums_kernel(const __grid_constant__ MapperGroup g, int uniq)
+{
+    const MapperSeg& s = g.seg[blockIdx.x];
+    if (s.n > 0) scan_tile_sums(uniq ? s.tiles_uniq : s.tiles_new, (s.n + kScanTile - 1) / kScanTile, nullptr);
+}
 static __global__ void __launch_bounds__(kScanThreads) group_new_reduce_kernel(const __grid_constant__ MapperGroup g)
 {
     const MapperSeg& s = g.seg[blockIdx.y];
     group_scan_reduce(WonBidIn{s.m.table, s.ent, s.miss}, s.n, s.tiles_new);
 }
-static __global__ void __launch_bounds__(kScanThreads) group_new_assign_kernel(const __grid_constant__ MapperGroup g)
+static __global__ void __launch_bounds__(kScanThreads) group_new_assign_kernel(const __grid_constant__ MapperGroup g, int fold)
 {
     const MapperSeg& s = g.seg[blockIdx.y];
     group_scan_apply(WonBidIn{s.m.table, s.ent, s.miss}, MapperAssignOut{s.m, s.ids, s.ent, s.status}, s.n, s.tiles_new,
-                     s.totals);
+                     fold, s.totals);
 }
 static __global__ void __launch_bounds__(256) group_readback_kernel(const __grid_constant__ MapperGroup g)
 {
@@ -461,10 +464,11 @@ static __global__ void __launch_bounds__(kScanThreads) group_uniq_reduce_kernel(
     const MapperSeg& s = g.seg[blockIdx.y];
     group_scan_reduce(HoldsMarkIn{s.slots, s.m.mark, s.m.init_max_index}, s.n, s.tiles_uniq);
 }
-static __global__ void __launch_bounds__(kScanThreads) group_uniq_rank_kernel(const __grid_constant__ MapperGroup g)
+static __global__ void __launch_bounds__(kScanThreads) group_uniq_rank_kernel(const __grid_constant__ MapperGroup g, int fold)
 {
     const MapperSeg& s = g.seg[blockIdx.y];
-    group_scan_apply(HoldsMarkIn{s.slots, s.m.mark, s.m.init_max_index}, RankOut{s.rank}, s.n, s.tiles_uniq, s.totals + 1);
+    group_scan_apply(HoldsMarkIn{s.slots, s.m.mark, s.m.init_max_index}, RankOut{s.rank}, s.n, s.tiles_uniq, fold,
+                     s.totals + 1);
 }
 // a table's unique slots start where those of the tables before it end
 static __global__ void __launch_bounds__(256) group_uniq_write_kernel(const __grid_constant__ MapperGroup g,
@@ -514,11 +518,14 @@ static int mapper_group_run(const MapperGroup& g, int tables, int64_t max_n, int
     const dim3 probe(static_cast<unsigned>(grid_for(n, 256 / kProbeLanes)), y), flat(static_cast<unsigned>(grid_for(n, 256)), y),
         tiles(static_cast<unsigned>(scan_num_tiles(n)), y);
     group_find_or_claim_kernel<<<probe, 256, 0, st>>>(g);
+    const int fold = tiles.x <= kScanFoldTiles ? 1 : 0;
     group_new_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g);
-    group_new_assign_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    if (!fold) group_tile_sums_kernel<<<y, 1024, 0, st>>>(g, 0);
+    group_new_assign_kernel<<<tiles, kScanThreads, 0, st>>>(g, fold);
     group_readback_kernel<<<flat, 256, 0, st>>>(g);
     group_uniq_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g);
-    group_uniq_rank_kernel<<<tiles, kScanThreads, 0, st>>>(g);
+    if (!fold) group_tile_sums_kernel<<<y, 1024, 0, st>>>(g, 1);
+    group_uniq_rank_kernel<<<tiles, kScanThreads, 0, st>>>(g, fold);
     group_uniq_write_kernel<<<flat, 256, 0, st>>>(g, unique, unique_ids, unique_offset);
     group_uniq_reset_kernel<<<flat, 256, 0, st>>>(g, status_out);
     RECSDK_CUDA_CHECK_LAUNCH();

@@ -97,8 +97,7 @@ static __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const 
 }
 
 // In place exclusive scan of `m` tile sums by one block; total -> *total_out (int64, optional).
-static __global__ void __launch_bounds__(1024) scan_tile_sums_kernel(int* __restrict__ tile_sums, int64_t m,
-                                                              int64_t* __restrict__ total_out)
+__device__ __forceinline__ void scan_tile_sums(int* __restrict__ tile_sums, int64_t m, int64_t* __restrict__ total_out)
 {
     __shared__ int sm[33];
     int carry = 0;
@@ -111,6 +110,11 @@ static __global__ void __launch_bounds__(1024) scan_tile_sums_kernel(int* __rest
         carry += total;
     }
     if (threadIdx.x == 0 && total_out != nullptr) *total_out = carry;
+}
+static __global__ void __launch_bounds__(1024) scan_tile_sums_kernel(int* __restrict__ tile_sums, int64_t m,
+                                                              int64_t* __restrict__ total_out)
+{
+    scan_tile_sums(tile_sums, m, total_out);
 }
 
 // Up to this many tiles the apply kernels fold the scan of the tile sums into themselves (every block adds up the

@@ -192,6 +192,31 @@ def test_mappers_together_equal_one_by_one(per_table, shared):
     assert [m.size() for m in together] == [m.size() for m in single]
 
 
+# segments on either side of the number of scan tiles (1024 of 2048 ids) up to which the offsets are added up tile by tile
+@pytest.mark.parametrize("long", [1024 * 2048, 1024 * 2048 + 1, 5_000_000])
+def test_mapper_segments_of_many_tiles(long):
+    from recsdk_b200 import IdsMapper
+
+    per_table = [3_000, long, 0, 2_049]
+    offs = np.concatenate([[0], np.cumsum(per_table)]).astype(np.int64)
+    n, T = int(offs[-1]), len(per_table)
+    ids = np.random.default_rng(long).integers(0, long // 3, n)
+    hi, uq, uid, inv = (torch.zeros(n, dtype=torch.int64, device=DEV) for _ in range(4))
+    uo = torch.zeros(T + 1, dtype=torch.int64, device=DEV)
+    IdsMapper.parallel_ids2indices_unique_out([IdsMapper(max(k, 16)) for k in per_table], _t(ids), hi, offs, uq, uid, inv, uo)
+    hi, uid, inv, uo = (x.cpu().numpy() for x in (hi, uid, inv, uo))
+    for t in range(T):
+        seg = ids[offs[t]:offs[t + 1]]
+        keys, first, which = np.unique(seg, return_index=True, return_inverse=True)
+        come = np.argsort(first)  # keys get slots, and stand in the unique list, in the order they come
+        slot = np.empty(keys.size, np.int64)
+        slot[come] = np.arange(keys.size)
+        assert uo[t + 1] - uo[t] == keys.size
+        np.testing.assert_array_equal(uid[uo[t]:uo[t + 1]], keys[come])
+        np.testing.assert_array_equal(hi[offs[t]:offs[t + 1]], slot[which])
+        np.testing.assert_array_equal(inv[offs[t]:offs[t + 1]], slot[which])
+
+
 def test_mappers_together_report_the_table_that_failed():
     from recsdk_b200 import IdsMapper
 
