@@ -48,10 +48,10 @@ constexpr int kChunk = 64;  // the only non-zero reduce_chunk supported
 // Small batches take as long as the chain of the longest direct run, large ones hide it behind other rows and pay for
 // every slot.  Chunk sums and row update together, us, with thresholds 8 / 16 / 64: 32768 log-uniform ids over 400000
 // rows of 8 floats 29 / 31 / 37; 131072 of 32 floats 37 / 37 / 41; training steps of 11 tables, 330 K ids, MEAN 202 / 198 /
-// 210 and of 205 K ids unpooled 235 / 235 / 243; 524288 uniform ids of 32 floats 80 / 74 / 75; 2^20 of 128 floats 308 / 303 /
-// 303, and the plan of 2^20 log-uniform ids 98 / 90 / 82.
+// 210 and of 205 K ids unpooled 235 / 235 / 243; 524288 log-uniform ids of 128 floats 120 / 119 / 110, uniform ones of 32
+// floats 80 / 74 / 75; the plan of 2^20 log-uniform ids 98 / 90 / 82.
 constexpr int kDirectMax = kChunk;
-constexpr int64_t kDirect8N = int64_t(1) << 17, kDirect16N = int64_t(1) << 19;
+constexpr int64_t kDirect8N = int64_t(1) << 17, kDirect16N = int64_t(3) << 17;
 static inline int direct_max_for(int64_t n) { return n <= kDirect8N ? 8 : (n <= kDirect16N ? 16 : kDirectMax); }
 // Slots of the partial buffer / chunk descriptors that n index positions can need with one threshold for direct runs.
 static inline size_t chunk_slots(int64_t n, int direct_max)

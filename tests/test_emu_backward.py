@@ -49,7 +49,7 @@ def test_runs_worth_a_kernel_of_their_own(emu, rows, dim, chunks, saves):
 
 
 # measured: the threshold for direct runs that took the least time, plan included
-@pytest.mark.parametrize("n,threshold", [(8_192, 8), (131_072, 8), (330_000, 16), (524_288, 16), (1 << 20, 64), (1 << 21, 64)])
+@pytest.mark.parametrize("n,threshold", [(8_192, 8), (131_072, 8), (330_000, 16), (524_288, 64), (1 << 20, 64), (1 << 21, 64)])
 def test_direct_run_threshold(emu, n, threshold):
     assert emu.emu_direct_max(n) == threshold
 
@@ -58,7 +58,7 @@ def test_chunk_slots_serve_every_smaller_batch(emu):
     sizes = sorted({max(1, (1 << k) + d) for k in range(0, 24) for d in (-1, 0, 1)} | {330_000, 700_000})
     need = [max(m // 64 + m // (emu.emu_direct_max(m) + 1) for m in sizes if m <= n) for n in sizes]
     assert all(emu.emu_chunk_slots_cap(n) >= k for n, k in zip(sizes, need))
-    assert emu.emu_chunk_slots_cap(1 << 20) <= (1 << 20) // 24  # one threshold of 8 up to 2^20 ids: 133 K slots
+    assert emu.emu_chunk_slots_cap(1 << 20) <= (1 << 20) // 30  # one threshold of 8 up to 2^20 ids: 133 K slots
 
 
 def _ptr(a):
