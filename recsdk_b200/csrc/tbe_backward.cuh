@@ -472,13 +472,15 @@ __device__ __forceinline__ bool vec_ok_for(const BwdParams& p, int64_t wofs, int
 }
 
 // ---------------------------------------------------------------------------- 4b. chunk sums
-// Narrow rows (G <= 8): eight tags per lane and 16 row loads in flight, two blocks per SM.  Wide rows: one tag per
+// Narrow rows (G <= 8): several tags per lane and 16 row loads in flight, two blocks per SM.  Wide rows: one tag per
 // lane, eight row loads, four blocks (64 registers) -- there the warps provide the bytes in flight, and 64-float rows
-// took 787 us with four tags per lane and three blocks against 612 with four.
+// took 787 us with four tags per lane and three blocks against 612 with four.  G == 8 takes four tags per lane: with
+// eight, 32-float rows took longer wherever the batch is small (sums and update of 8192 ids, half of them one row: 25 us
+// against 21) and 2^21 log-uniform ids 163 us against 147.
 template <int G>
 __host__ __device__ constexpr int chunk_tags()
 {
-    return G == 1 ? 16 : (G <= 8 ? 8 : 1);
+    return G == 1 ? 16 : (G < 8 ? 8 : (G == 8 ? 4 : 1));
 }
 __host__ __device__ constexpr int chunk_blocks(int G) { return G <= 8 ? 2 : 4; }
 __host__ __device__ constexpr int chunk_loads(int G) { return G <= 8 ? 16 : 8; }
