@@ -74,15 +74,18 @@ static inline size_t chunk_slots_cap(int64_t n)
 // it.  The order of that sum is fixed, so its adds are one chain, but its loads need not be: a group of the row update
 // keeps four in flight beside its table row, a warp of that kernel 224.  Hottest row of 20 M Zipf(1.2) ids in 26 tables,
 // about 2600 chunks: the row update as a whole took 1027 us with its chain in it, 724 without, and this kernel 60.
-// A chain of c chunks takes 0.15 to 0.4 us a chunk and is hidden while the update of all the other rows, about 1 to 1.6 us
-// per MB of them, takes longer: a run is listed for the kernel from kLongChunks + 4 per MB of updated rows on.
-// With every run above 64 chunks listed, chunk sums and update of 524288 log-uniform ids of 128 floats (64 MB of rows,
-// hottest row 440 chunks) took 122 us, with none 110; of 131072 ids of 64 floats 41 and 35; of 2^20 ids of 64 floats
-// (52 MB, 884 chunks) 139 and 180; of 65536 ids half of which are one row, 8 floats, 41 and 58.
+// A chain is hidden while the update of the rows that come after it takes longer, which depends on the bytes of the rows:
+// chunk sums and update of 524288 log-uniform ids (hottest row 440 chunks), every run above 224 chunks listed / none,
+// rows of 32 floats 52 / 72 us, of 128 floats 123 / 113; of 330 K ids of 128 floats (278 chunks) 90 / 82.  So a run is
+// listed from 224 chunks + 5 per MB of updated rows on, but from 480 at the latest: the hot rows of several tables come up
+// anywhere, also late, and then nothing hides them.  Training step of 20 M ids in 26 tables, us, by the number of chunks
+// from which runs are listed: 64 3001, 224 2975, 666 2990, 1990 3086, never 3250.  Steps on tables of mixed widths and on
+// sequences, whose runs are shorter: 64 198 and 242, 224 193 and 234.
 constexpr int kLongChunks = 224;
-__host__ __device__ __forceinline__ int64_t long_run_chunks(int64_t rows, int32_t max_D)
+__host__ __device__ __forceinline__ int long_run_chunks(int64_t rows, int32_t max_D)
 {
-    return kLongChunks + ((rows * max_D) >> 18) * 4;
+    const int64_t more = ((rows * max_D) >> 18) * 5;
+    return kLongChunks + (more < 256 ? static_cast<int>(more) : 256);
 }
 // Runs that can be longer than that: n positions hold at most n / (kLongChunks * kChunk) of them.
 static inline size_t long_runs_cap(int64_t n) { return static_cast<size_t>(n > 0 ? n : 0) / (kLongChunks * kChunk) + 1; }

@@ -97,4 +97,4 @@ extern "C" int emu_tbe_backward(const float* grad, float* w, float* m1, float* m
 
 extern "C" int emu_direct_max(int64_t n) { return direct_max_for(n); }
 extern "C" int64_t emu_chunk_slots_cap(int64_t n) { return static_cast<int64_t>(chunk_slots_cap(n)); }
-extern "C" int64_t emu_long_run_chunks(int64_t rows, int32_t max_D) { return long_run_chunks(rows, max_D); }
+extern "C" int emu_long_run_chunks(int64_t rows, int32_t max_D) { return long_run_chunks(rows, max_D); }
