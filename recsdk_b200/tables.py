@@ -123,6 +123,9 @@ class IdsMapper:
     def parallel_ids2indices_unique_out(mappers: Sequence["IdsMapper"], ids, hash_indices, offsets, unique,
                                         unique_ids, unique_inverse, unique_offset, check: bool = True) -> None:
         """ids_mapper.cpp:227-285: one mapper per table; the tables' phases run together, one launch per phase."""
+        T = len(mappers)
+        if T == 0:
+            return
         _chk(ids, torch.int64, "globalIds")
         _chk(hash_indices, torch.int64, "hashIndices")
         _chk(unique, torch.int64, "unique")
@@ -130,9 +133,6 @@ class IdsMapper:
         _chk(unique_inverse, torch.int64, "uniqueInverse")
         _chk(unique_offset, torch.int64, "uniqueOffset")
         offs = [int(o) for o in (offsets.tolist() if isinstance(offsets, torch.Tensor) else offsets)]
-        T = len(mappers)
-        if T == 0:
-            return
         if not (len(offs) - 1 > T - 1):
             raise RuntimeError("offset must be equal to table size + 1")
         ws = [m._workspace_for(offs[t + 1] - offs[t]) for t, m in enumerate(mappers)]

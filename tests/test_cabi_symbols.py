@@ -64,3 +64,12 @@ def test_cpu_tensors_are_rejected():
     with pytest.raises(RuntimeError, match="CUDA tensor"):
         ops.tbe_forward(w, torch.zeros(1, dtype=torch.int64), torch.tensor([0, 4], dtype=torch.int32),
                         torch.zeros(2, dtype=torch.int64), torch.tensor([0, 1, 2]), 4, 4, 0)
+
+
+def test_no_mappers_no_checks():
+    """A batch without hash-keyed tables asks nothing of its tensors."""
+    import torch
+    from recsdk_b200 import IdsMapper
+
+    none = torch.zeros(0)
+    assert IdsMapper.parallel_ids2indices_unique_out([], none, none, [0], none, none, none, none) is None
