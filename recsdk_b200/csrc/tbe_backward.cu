@@ -5,16 +5,18 @@
 //   1. expand   : every index position p -> (key, val); key identifies the row
 //                 (hash_size_cumsum[t] + idx, or inverse[p] + unique_offsets[t]),
 //                 val packs (feature, sample) of the bag whose gradient row p takes.
-//                 The kernel also counts the first sort pass's histogram.
+//                 Below 2^20 pairs the kernel also counts the first pass's histogram.
 //   2. sort     : stable LSD radix sort of the pairs by key (prims.cuh), per pass a
-//                 scan and a scatter that counts the next pass's histogram.  Equal
-//                 keys stay in ascending position order -> fixed reduction order.
+//                 scan and a scatter that counts the next pass's histogram, or from
+//                 2^20 pairs on three kernels over large tiles.  Equal keys stay in
+//                 ascending position order -> fixed reduction order.
 //   3. runs     : head flags (computed inside the scan) -> run starts, U.
 //   4. records  : one thread per unique row resolves everything the update needs
 //                 (row address, first gradient row address, run, width) into a
-//                 32-byte record; runs longer than C reserve chunk slots.
-//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp), and for runs of
-//                 many chunks the total of those.
+//                 32-byte record; runs longer than direct_max reserve chunk slots.
+//                 (1. to 4. are one kernel of one block up to 8192 positions.)
+//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp), and
+//                 for runs of many chunks the total of those.
 //   5. update   : G lanes per unique row: record (fetched one row ahead) -> w / m1 /
 //                 m2 / first gradient row in one wave of loads -> remaining gradient
 //                 rows or chunk sums in order -> optimizer -> one write of w / m1 /
@@ -29,7 +31,10 @@
 #ifndef RECSDK_EMULATE
 namespace recsdk {
 // ---------------------------------------------------------------------------- host side
-constexpr int64_t kLongRunMinIds = 32768;
+// Below this many ids long_run_kernel is not launched: a run of more than kLongChunks chunks would be over a fifth of
+// them.  The launch takes 2 us on the device (131072 uniform ids of 8 floats 12.4 -> 14.5 us of sums and update); 65536 ids
+// half of which are one row take 41 us with it and 58 without.
+constexpr int64_t kLongRunMinIds = 65536;
 
 struct BwdWorkspace {
     void *keys_a, *keys_b;
@@ -175,7 +180,6 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     p.counters = ws.counters;
     p.chunk_desc = ws.desc;
     p.partial = ws.partial;
-    // below this many ids hardly any row is that long and the launch costs more than its chain
     p.long_runs = (N >= kLongRunMinIds && p.chunk > 0) ? 1 : 0;
     p.long_list = ws.long_list;
     const int vec_per_row = (a->max_D + 3) / 4;

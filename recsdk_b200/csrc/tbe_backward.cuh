@@ -5,15 +5,18 @@
 //   1. expand   : every index position p -> (key, val); key identifies the row
 //                 (hash_size_cumsum[t] + idx, or inverse[p] + unique_offsets[t]),
 //                 val packs (feature, sample) of the bag whose gradient row p takes.
-//                 The kernel also counts the first sort pass's histogram.
+//                 Below 2^20 pairs the kernel also counts the first pass's histogram.
 //   2. sort     : stable LSD radix sort of the pairs by key (prims.cuh), per pass a
-//                 scan and a scatter that counts the next pass's histogram.  Equal
-//                 keys stay in ascending position order -> fixed reduction order.
+//                 scan and a scatter that counts the next pass's histogram, or from
+//                 2^20 pairs on three kernels over large tiles.  Equal keys stay in
+//                 ascending position order -> fixed reduction order.
 //   3. runs     : head flags (computed inside the scan) -> run starts, U.
 //   4. records  : one thread per unique row resolves everything the update needs
 //                 (row address, first gradient row address, run, width) into a
-//                 32-byte record; runs longer than C reserve chunk slots.
-//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp).
+//                 32-byte record; runs longer than direct_max reserve chunk slots.
+//                 (1. to 4. are one kernel of one block up to 8192 positions.)
+//   4b. partial : chunk sums of the long runs (keeps Zipf-hot rows off one warp), and
+//                 for runs of many chunks the total of those.
 //   5. update   : G lanes per unique row: record (fetched one row ahead) -> w / m1 /
 //                 m2 / first gradient row in one wave of loads -> remaining gradient
 //                 rows or chunk sums in order -> optimizer -> one write of w / m1 /

@@ -87,8 +87,9 @@ def test_backward_long_runs_of_mixed_widths(dims, opt):
     from recsdk_b200 import ops
 
     rng = np.random.default_rng(sum(dims))
-    B, per_bag = 2_000, 16
+    B, per_bag = 2_000, 17
     n, total = 2 * B * per_bag, sum(dims)
+    assert n > 65_536  # from there on that kernel is launched
     indices = np.where(rng.random(n) < 0.9, 1, rng.integers(0, 3, n))
     offsets = np.arange(2 * B + 1, dtype=np.int64) * per_bag
     wo, do, hs = np.array([0, 3 * dims[0]], np.int64), np.array([0, dims[0], total], np.int32), np.array([0, 3, 6], np.int64)
