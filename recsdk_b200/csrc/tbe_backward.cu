@@ -31,9 +31,9 @@
 #ifndef RECSDK_EMULATE
 namespace recsdk {
 // ---------------------------------------------------------------------------- host side
-// Below this many ids long_run_kernel is not launched: a run of more than kLongChunks chunks would be over a fifth of
-// them.  The launch takes 2 us on the device (131072 uniform ids of 8 floats 12.4 -> 14.5 us of sums and update); 65536 ids
-// half of which are one row take 41 us with it and 58 without.
+// Below this many ids long_run_kernel is not launched: a run long enough for it would be over a fifth of them.  The
+// launch takes 2 us on the device (131072 uniform ids of 8 floats 12.4 -> 14.5 us of sums and update); 65536 ids half of
+// which are one row take 41 us with it and 58 without.
 constexpr int64_t kLongRunMinIds = 65536;
 
 struct BwdWorkspace {
@@ -189,7 +189,7 @@ static int run_backward(const recsdk_tbe_backward_args* a, BwdParams p, const Bw
     } else if (do_plan) {
         // The plan needs the indices and the LAYOUT of the gradient, not the gradient: it can run ahead, on
         // another stream, while the forward of the same batch (or the dense part) runs.
-        cudaMemsetAsync(ws.counters, 0, 8 * sizeof(int64_t), st);  // {U, chunks, indices in chunked runs, unaligned columns, ...}
+        cudaMemsetAsync(ws.counters, 0, 8 * sizeof(int64_t), st);  // {U, chunks, indices in chunked runs, unaligned columns, long runs, chunks of the longest}
         // 1. expand; unless the sort is the one for large inputs it also fills the histogram of the first pass
         const bool big = radix_sort_is_big<KeyT>(N, key_bits);
         RadixFusedPlan plan{};

@@ -78,17 +78,19 @@ static inline size_t chunk_slots_cap(int64_t n)
 // keeps four in flight beside its table row, a warp of that kernel 224.  Hottest row of 20 M Zipf(1.2) ids in 26 tables,
 // about 2600 chunks: the row update as a whole took 1027 us with its chain in it, 724 without, and this kernel 60.
 // A chain is hidden while the update of the rows that come after it takes longer, which depends on the bytes of the rows:
-// chunk sums and update of 524288 log-uniform ids (hottest row 440 chunks), every run above 224 chunks listed / none,
-// rows of 32 floats 52 / 72 us, of 128 floats 123 / 113; of 330 K ids of 128 floats (278 chunks) 90 / 82.  So a run is
-// listed from 224 chunks + 5 per MB of updated rows on, but from 480 at the latest: the hot rows of several tables come up
-// anywhere, also late, and then nothing hides them.  Training step of 20 M ids in 26 tables, us, by the number of chunks
-// from which runs are listed: 64 3001, 224 2975, 666 2990, 1990 3086, never 3250.  Steps on tables of mixed widths and on
-// sequences, whose runs are shorter: 64 198 and 242, 224 193 and 234.
-constexpr int kLongChunks = 224;
+// chunk sums and update of 524288 log-uniform ids (hottest row 440 chunks), every run above 224 chunks taken / none,
+// rows of 32 floats 52 / 72 us, of 128 floats 123 / 113; of 330 K ids of 128 floats (278 chunks) 90 / 82.  So the kernel works
+// when the longest run of the batch has more than 224 chunks + 5 per MB of updated rows, but from 480 at the latest: the
+// hot rows of several tables come up anywhere, also late, and then nothing hides them.  When it works it takes every run
+// above kLongChunks: one more costs it nothing, as it lasts as long as its longest.  Training step of 20 M ids in 26
+// tables, us, by the number of chunks from which runs are taken: 64 3001, 224 2975, 666 2990, 1990 3086, never 3250; row update of
+// 215 K Zipf(1.16) ids of 16 floats, whose hottest row has 600: 64 11.3, 224 15.9.  Steps on tables of mixed widths and on
+// sequences, whose longest runs are about 100: 64 198 and 242, never 193 and 234.
+constexpr int kLongChunks = 112;
 __host__ __device__ __forceinline__ int long_run_chunks(int64_t rows, int32_t max_D)
 {
     const int64_t more = ((rows * max_D) >> 18) * 5;
-    return kLongChunks + (more < 256 ? static_cast<int>(more) : 256);
+    return 224 + (more < 256 ? static_cast<int>(more) : 256);
 }
 // Runs that can be longer than that: n positions hold at most n / (kLongChunks * kChunk) of them.
 static inline size_t long_runs_cap(int64_t n) { return static_cast<size_t>(n > 0 ? n : 0) / (kLongChunks * kChunk) + 1; }
@@ -130,16 +132,21 @@ struct BwdParams {
     // (buffer number << kLocShardShift) | element offset inside that buffer; the buffers may be peer mappings.
     float* dst_ptrs[RECSDK_MAX_SHARDS];
     int32_t direct_max;  // runs longer than this go through the chunk-sum kernel
-    // != 0: runs of more than long_run_chunks() chunks are listed in long_list (counters[4] of them) and long_run_kernel
-    // leaves their total in their first chunk slot before the row update reads it
+    // != 0: runs of more than kLongChunks chunks are listed in long_list (counters[4] of them, the longest of counters[5]
+    // chunks); if that is more than long_run_chunks(), long_run_kernel leaves their totals in their first chunk slots
+    // before the row update reads them
     int32_t long_runs;
     int* __restrict__ long_list;
 };
 
-// Of a run of `chunks` chunks among `rows` distinct rows.
-__device__ __forceinline__ bool is_long_run(const BwdParams& p, int chunks, int64_t rows)
+// Does long_run_kernel work on this batch, is a run of `chunks` chunks one of its?  (p.counters as the plan left them.)
+__device__ __forceinline__ bool long_runs_taken(const BwdParams& p)
 {
-    return p.long_runs != 0 && chunks > kLongChunks && chunks > long_run_chunks(rows, p.max_D);
+    return p.counters[5] > long_run_chunks(p.counters[0], p.max_D);
+}
+__device__ __forceinline__ bool is_long_run(const BwdParams& p, int chunks)
+{
+    return p.long_runs != 0 && chunks > kLongChunks && long_runs_taken(p);
 }
 
 // Internal "optimizer" of the row-update kernels: no table is read, the summed gradient of the row is stored.
@@ -620,8 +627,10 @@ __device__ __forceinline__ RunMeta make_run_meta(const BwdParams& p, int64_t r, 
                                                     static_cast<unsigned long long>(c)));
         atomicAdd(reinterpret_cast<unsigned long long*>(counters + 2), static_cast<unsigned long long>(len));
         m.chunk_base = base;
-        if (is_long_run(p, c, counters[0]))
+        if (p.long_runs != 0 && c > kLongChunks) {
             p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(counters + 4), 1ull)] = static_cast<int>(r);
+            atomicMax(reinterpret_cast<unsigned long long*>(counters + 5), static_cast<unsigned long long>(c));
+        }
         for (int k = 0; k < c; ++k) {
             const int b0 = rs + k * step;
             desc[base + k] = make_int2(b0, b0 + step < re ? b0 + step : re);
@@ -733,7 +742,7 @@ __global__ void __launch_bounds__(kSmallThreads) plan_small_kernel(BwdParams p, 
     }
 }
 // ---------------------------------------------------------------------------- 4c. totals of the longest runs
-// One warp per (listed run, see long_run_chunks(), 32 columns): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
+// One warp per (listed run, 32 columns), if the batch needs it (long_run_chunks()): lane = column, chunk sums added in chunk order from 0.0f; the total takes the
 // place of the run's first chunk sum (no other warp reads these columns of this run).  The chunk sums come through a
 // ring of kLongStages shared-memory stages of 32 rows, filled by asynchronous copies, so 224 rows are in flight
 // whatever the registers; each lane copies and reads its own column, so a stage needs no barrier.
@@ -745,7 +754,7 @@ static __global__ void __launch_bounds__(kLongWarps * 32) long_run_kernel(BwdPar
     __shared__ float ring[kLongWarps][kLongStages][kLongRows][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int slabs = (p.max_D + 31) / 32;
-    const int64_t items = p.counters[4] * slabs;
+    const int64_t items = long_runs_taken(p) ? p.counters[4] * slabs : 0;
     for (int64_t w = static_cast<int64_t>(blockIdx.x) * kLongWarps + warp; w < items;
          w += static_cast<int64_t>(gridDim.x) * kLongWarps) {
         const RunMeta* m = meta + p.long_list[w / slabs];
@@ -788,7 +797,7 @@ __device__ __forceinline__ void row_gradient(const BwdParams& p, const RunMeta& 
     const bool chunked = m.chunk_base >= 0;
     if (chunked) {
         int nc = chunks_of_run(m.len, p.chunk);
-        if (is_long_run(p, nc, p.counters[0])) nc = 1;  // long_run_kernel left the total in the first slot
+        if (is_long_run(p, nc)) nc = 1;  // long_run_kernel left the total in the first slot
         int c = 0;
         for (; c + 4 <= nc; c += 4) {
             typename V::T v[4][K];

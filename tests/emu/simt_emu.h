@@ -47,6 +47,8 @@ static inline unsigned long long atomicCAS(unsigned long long* p, unsigned long 
 { std::lock_guard<std::mutex> l(g_atomic_mu); unsigned long long o = *p; if (o == cmp) *p = v; return o; }
 static inline unsigned long long atomicAdd(unsigned long long* p, unsigned long long v)
 { std::lock_guard<std::mutex> l(g_atomic_mu); unsigned long long o = *p; *p = o + v; return o; }
+static inline unsigned long long atomicMax(unsigned long long* p, unsigned long long v)
+{ std::lock_guard<std::mutex> l(g_atomic_mu); unsigned long long o = *p; if (v > o) *p = v; return o; }
 
 // ---- collective rendezvous keyed by (warp, mask)
 struct Rendezvous {

@@ -59,11 +59,11 @@ def test_backward_plan_sizes(n, bits):
     _backward_equals_oracle(rng.integers(0, 60_000, n), 60_000, 4, min(n, 5_000), bits)
 
 
-# runs around the direct / chunked borders (8, 16, 64 by the size of the batch), a chunk, the border above which a run's
-# chunk sums get their own kernel (224 chunks with so few rows), and that kernel's ring of 256 chunk sums taken around
-# more than once
+# runs around the direct / chunked borders (8, 16, 64 by the size of the batch), a chunk, the borders above which the sum of
+# a run's chunk sums gets its own kernel (112 chunks, if the longest run has more than 224), and that kernel's ring of 256
+# chunk sums taken around more than once
 RUNS = [1, 2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 128, 129, 4095, 4096, 4097, 4161, 14_000, 16 * 64, 17 * 64 + 1]
-LONG_RUNS = [224 * 64, 224 * 64 + 1, 256 * 64, 256 * 64 + 1, 40_000]
+LONG_RUNS = [112 * 64, 112 * 64 + 1, 224 * 64, 224 * 64 + 1, 256 * 64, 256 * 64 + 1, 40_000]
 
 
 @pytest.mark.parametrize("dim", [4, 8, 16, 32, 36, 64, 128, 18])
@@ -77,6 +77,7 @@ def test_backward_run_lengths(dim):
 
     assert check(RUNS[:12], 301, 1) < 8192
     assert 32_768 < check(RUNS, 3_001, 0) < 1 << 17
+    assert 65_536 < check(RUNS + LONG_RUNS[:3] + [9_000, 10_000], 3_001, 0) < 1 << 17  # 224 chunks: the kernel stays idle
     assert 1 << 17 < check(RUNS + LONG_RUNS, 3_001, 0) < 3 << 17
 
 
