@@ -55,6 +55,18 @@ def seeded_rows():
     return [int(r) for r in np.round(10 ** rng.uniform(math.log10(1e3), math.log10(4e7), N_TABLES)).astype(np.int64)]
 
 
+def backward_launches(n, bags, key_bits):
+    """Kernels of one fused backward (chunks of 64): the plan, chunk sums, totals of hot rows, row update."""
+    if n <= 8192 and bags <= 8192:
+        plan = 1
+    else:
+        passes = min(math.ceil(key_bits / digit) for digit in (8, 9, 10))
+        per_pass = 3 if n >= 1 << 20 else 2  # histogram + scan + scatter, or scan + scatter
+        run_scan = 3 if n > 1024 * 2048 else 2
+        plan = 1 + passes * per_pass + run_scan + 1  # expand, sort, run starts, records
+    return plan + 1 + (1 if n >= 65536 else 0) + 1
+
+
 def measured_peak_gbs():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -396,9 +408,7 @@ def run_ours(args):
         step_bytes = (16 * N + 8 * U) + (N * (8 + 4 * DIM) + 8 * (N + 1) + 4 * DIM * N) + \
                      (4 * DIM * N + 8 * N + 8 * U + U * 4 * DIM * 2 * (1 + S))
         bits = module.total_hash_size_bits
-        passes = min(math.ceil(bits / 8), math.ceil(bits / 9))  # the sort takes 9-bit digits when that saves a pass
-        # forward + expand, (scan + scatter) per sort pass, 3 run-scan kernels, records, partial sums, update
-        launches_per_step = 1 + (1 + 2 * passes + 3 + 1 + 1 + 1)
+        launches_per_step = 1 + backward_launches(N, N, bits)  # one id per bag
         line = {
             "metric": "embedding ids/sec (fwd+bwd+sparse Adam)",
             "value": value,
@@ -918,7 +928,7 @@ def run_tbe_config(args, name):
     e2e_ms, issue_ms = _time_loop(torch, step_e2e, args.steps, max(args.warmup, 3, args.steps))  # pool warm, see run_ours
     without_graph = None
     if name == "c1":
-        # the step is a dozen kernels of a few microseconds: replayed as ONE CUDA graph (static index / offset buffers
+        # the step is a few kernels of a few microseconds: replayed as ONE CUDA graph (static index / offset buffers
         # refilled every step: device-to-device for `value`, from pinned host memory for `e2e`)
         s_idx, s_offs = batches[0][0].clone(), batches[0][1].clone()
         graph = module.capture_step(s_idx, s_offs, out, grad)
@@ -963,11 +973,12 @@ def run_tbe_config(args, name):
         "e2e": {"value": N / (e2e_ms * 1e-3), "unit": "ids/s", "ms_per_step": e2e_ms, "host_enqueue_ms_per_step": issue_ms,
                 "h2d_bytes_per_step": int(host[0][0].numel() * 4 + host[0][1].numel() * 4),
                 "d2h_bytes_per_step": int(result_host.numel() * 4)},
-        "gpu_launches": (1 + 1 + 2 * 3 + 3 + 1 + 1 + 1) * args.steps,
+        "gpu_launches": (1 + backward_launches(N, bags, module.total_hash_size_bits)) * args.steps,
         "clocks": clocks,
     }
     if without_graph is not None:
-        line["config"]["step"] = "forward + fused backward captured once as a CUDA graph and replayed (13 kernels per replay)"
+        kernels = 1 + backward_launches(N, bags, module.total_hash_size_bits)
+        line["config"]["step"] = f"forward + fused backward captured once as a CUDA graph and replayed ({kernels} kernels per replay)"
         line["without_graph"] = without_graph
     if not args.no_cpu_baseline:
         line["cpu_baseline"] = _cpu_tbe_config(name, rows, D, B, alpha, max_len, args.cpu_budget)
